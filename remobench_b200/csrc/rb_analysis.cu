@@ -35,69 +35,150 @@ __device__ __forceinline__ bool leafA(const Dev& d, uint32_t node) {
     return (a.x & a.y & a.z & a.w & b.x & b.y & b.z & b.w) == -1;
 }
 
-// One level of the roll-up: leaves copy their accumulator; inner nodes add
-// their children, each re-based by its offset o (0 or half the parent) in the
-// parent's 2^(28 - L) grid: S1 += n o, S2_ab += o_a S1_b + o_b S1_a + n o_a o_b.
-__global__ void __launch_bounds__(256) k_roll_level(Dev d, RollSum* roll, uint32_t level) {
+// The roll-up: every node's sums over its subtree's leaves. With coordinates
+// taken from the root's origin they are plain additions, so a leaf's sums are
+// first re-based by its own origin O in the 2^28 grid: S1 += n O,
+// S2_ab += O_a S1_b + O_b S1_a + n O_a O_b, and k_analyze re-bases each node's
+// total back to the node's origin. Integers modulo 2^64 and 2^128: any order of
+// additions gives the same bits, and the totals fit.
+//
+// One launch for every level. A split hands its children eight consecutive ids
+// in octant order, so sibling group g is nodes 1 + 8 g .. 8 + 8 g and eight
+// lanes hold one group, each its node's sums. They go through shared memory so
+// that each lane adds up a share of the parent's words and writes it (a
+// butterfly of shuffles moves every word three times). A group whose members
+// are all leaves goes on to its parent's group; elsewhere the last of the
+// group's own leaves and its inner members to arrive does (rollArrive counts
+// them, and the one that goes on clears it). No block waits for another. Bound
+// by the longest chain of dependent round trips, one arrival and one read per
+// level of the tree, not by bytes (184 B read and written per node). Measured
+// at 31,497 nodes: 232 us as a launch per level (a pass over all nodes for each
+// of the 21, whatever the tree's depth), 40 us so; at 2,000 nodes 120 and
+// 27 us. Re-basing at every step of the chain instead: 59 and 33 us.
+constexpr uint32_t kRollThreads = 128;
+constexpr uint32_t kRollWords = sizeof(RollSum) / 8u;
+
+// r, relative to the origin of the node at `level` with coordinates N, to the
+// root's origin (up) or back (down).
+template <bool up>
+__device__ __forceinline__ void rollRebase(RollSum& r, uint32_t level, uint32_t X, uint32_t Y, uint32_t Z) {
+    const uint32_t sh = 28u - level;
+    const unsigned long long o[3] = {(unsigned long long)X << sh, (unsigned long long)Y << sh,
+                                     (unsigned long long)Z << sh};
+    const int pa[6] = {0, 0, 0, 1, 1, 2}, pb[6] = {0, 1, 2, 1, 2, 2};
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        u128 s2 = ((u128)r.s2[2 * k + 1] << 64) | r.s2[2 * k];
+        const u128 cross = (u128)o[pa[k]] * r.s1[pb[k]] + (u128)o[pb[k]] * r.s1[pa[k]];
+        const u128 square = (u128)(o[pa[k]] * o[pb[k]]) * r.n;
+        s2 = up ? s2 + cross + square : s2 - cross + square;
+        r.s2[2 * k] = (unsigned long long)s2;
+        r.s2[2 * k + 1] = (unsigned long long)(s2 >> 64);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) r.s1[k] = up ? r.s1[k] + r.n * o[k] : r.s1[k] - r.n * o[k];
+}
+
+__device__ __forceinline__ RollSum leafSums(const AccumI& a) {
+    RollSum r;
+    r.n = a.count;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        r.s1[k] = a.s1[k];
+        r.c1[k] = a.c1[k];
+        r.c2[k] = a.c2[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        r.s2[2 * k] = a.s2lo[k];
+        r.s2[2 * k + 1] = a.s2hi[k];
+    }
+    r.lastTouched = a.count ? a.lastTouchedBatch : 0u;
+    r.pad = 0;
+    return r;
+}
+
+// One more arrival: what the group's lanes wrote before it is visible to the
+// one that sees the last.
+__device__ __forceinline__ uint32_t arriveAcqRel(uint32_t* p) {
+    uint32_t old;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
+    return old;
+}
+
+__global__ void __launch_bounds__(kRollThreads) k_roll(Dev d, RollSum* roll, uint32_t* rollArrive,
+                                                       AnalysisCounters* ac) {
+    __shared__ unsigned long long s_words[kRollThreads / 8][8][kRollWords];
     const uint32_t nn = d.ctr->numNodes;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
-        if (d.level[i] != level) continue;
-        RollSum r;
-        if (leafA(d, i)) {
-            const AccumI& a = d.accum[i];
-            r.n = a.count;
-            for (int k = 0; k < 3; k++) r.s1[k] = a.s1[k];
-            for (int k = 0; k < 6; k++) {
-                r.s2[2 * k] = a.s2lo[k];
-                r.s2[2 * k + 1] = a.s2hi[k];
-            }
-            for (int k = 0; k < 3; k++) {
-                r.c1[k] = a.c1[k];
-                r.c2[k] = a.c2[k];
-            }
-            r.lastTouched = a.count ? a.lastTouchedBatch : 0u;
-            r.pad = 0;
-        } else {
-            unsigned long long cc1[3] = {0, 0, 0}, cc2[3] = {0, 0, 0};
-            u128 s1[3] = {0, 0, 0}, s2[6] = {0, 0, 0, 0, 0, 0};
-            u128 n = 0;
-            uint32_t lt = 0;
-            const uint32_t sh = 28u - (level + 1u);
-            for (int c = 0; c < 8; c++) {
-                const int32_t ci = d.child[i * 8u + c];
-                if (ci < 0) continue;
-                const RollSum& cr = roll[ci];
-                if (cr.n == 0) continue;
-                const u128 cn = cr.n;
-                const u128 o[3] = {(u128)((c >> 2) & 1) << sh, (u128)((c >> 1) & 1) << sh, (u128)(c & 1) << sh};
-                const u128 c1[3] = {cr.s1[0], cr.s1[1], cr.s1[2]};
-                n += cn;
-                for (int k = 0; k < 3; k++) s1[k] += c1[k] + cn * o[k];
-                const int pa[6] = {0, 0, 0, 1, 1, 2}, pb[6] = {0, 1, 2, 1, 2, 2};
-                for (int k = 0; k < 6; k++) {
-                    const u128 c2 = ((u128)cr.s2[2 * k + 1] << 64) | cr.s2[2 * k];
-                    s2[k] += c2 + o[pa[k]] * c1[pb[k]] + o[pb[k]] * c1[pa[k]] + cn * o[pa[k]] * o[pb[k]];
-                }
-                lt = cr.lastTouched > lt ? cr.lastTouched : lt;
-                for (int k = 0; k < 3; k++) {
-                    cc1[k] += cr.c1[k];
-                    cc2[k] += cr.c2[k];
-                }
-            }
-            for (int k = 0; k < 3; k++) {
-                r.c1[k] = cc1[k];
-                r.c2[k] = cc2[k];
-            }
-            r.n = (unsigned long long)n;
-            for (int k = 0; k < 3; k++) r.s1[k] = (unsigned long long)s1[k];
-            for (int k = 0; k < 6; k++) {
-                r.s2[2 * k] = (unsigned long long)s2[k];
-                r.s2[2 * k + 1] = (unsigned long long)(s2[k] >> 64);
-            }
-            r.lastTouched = lt;
-            r.pad = 0;
+    const uint32_t oct = threadIdx.x & 7u;
+    const unsigned gmask = 0xFFu << (threadIdx.x & 24u);
+    unsigned long long(*words)[kRollWords] = s_words[threadIdx.x >> 3];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *ac = AnalysisCounters{};
+        if (leafA(d, 0)) roll[0] = leafSums(d.accum[0]);  // its origin is the root's
+    }
+    // the words this lane adds up: lanes 0..5 a 128-bit sum of s2 and one of
+    // {n, s1}; lanes 6 and 7 the three of c1 or c2
+    const bool pair = oct < 6u;
+    const uint32_t w0 = pair ? 4u + 2u * oct : (oct == 6u ? 16u : 19u), w1 = w0 + 1u;
+    const uint32_t w2 = oct < 4u ? oct : w0 + 2u;
+    const bool third = oct < 4u || !pair;
+    const uint32_t groups = nn / 8u;  // the root, then eight nodes per split
+    for (uint32_t g0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; g0 < groups; g0 += (gridDim.x * blockDim.x) >> 3) {
+        uint32_t g = g0, node = 1u + 8u * g + oct;
+        bool leaf = leafA(d, node);
+        uint32_t parent = d.parent[node].x;
+        RollSum r = {};
+        if (leaf) {
+            r = leafSums(d.accum[node]);
+            rollRebase<true>(r, d.level[node], d.nodeX[node], d.nodeY[node], d.nodeZ[node]);
+            roll[node] = r;
         }
-        roll[i] = r;
+        // a collapsed node's former children hang off nothing
+        const bool attached = d.child[parent * 8u + oct] == (int32_t)node;
+        if (__ballot_sync(gmask, attached) != gmask) continue;
+        __syncwarp(gmask);
+        const bool whole = __ballot_sync(gmask, leaf) == gmask;
+        for (bool start = true;; start = false) {
+            if (start && whole) {
+                const unsigned long long* q = reinterpret_cast<const unsigned long long*>(&r);
+#pragma unroll
+                for (uint32_t k = 0; k < kRollWords; k++) words[oct][k] = q[k];
+            } else {
+                uint32_t arrived = 0;
+                if (oct == 0u) arrived = arriveAcqRel(&rollArrive[g]) + 1u;
+                arrived = __shfl_sync(gmask, arrived, 0, 8);
+                const uint32_t inner = __popc(__ballot_sync(gmask, !leaf));
+                if (arrived != inner + 1u) break;
+                if (oct == 0u) rollArrive[g] = 0u;
+                const unsigned long long* p = reinterpret_cast<const unsigned long long*>(&roll[node]);
+#pragma unroll
+                for (uint32_t k = 0; k < kRollWords; k++) words[oct][k] = __ldcg(p + k);
+            }
+            __syncwarp(gmask);
+            unsigned long long a = 0, b = 0, e = 0, lt = 0;
+#pragma unroll
+            for (uint32_t m = 0; m < 8u; m++) {
+                const unsigned long long va = words[m][w0];
+                a += va;
+                b += words[m][w1] + (pair && a < va ? 1ull : 0ull);
+                e += words[m][w2];
+                lt = max(lt, words[m][22]);
+            }
+            unsigned long long* out = reinterpret_cast<unsigned long long*>(&roll[parent]);
+            out[w0] = a;
+            out[w1] = b;
+            if (third) out[w2] = e;
+            if (oct == 5u) out[22] = lt;  // the newest batch; pad is zero
+            if (parent == 0u) break;
+            // the group above: what does not depend on its other members
+            g = (parent - 1u) >> 3;
+            node = 1u + 8u * g + oct;
+            leaf = leafA(d, node);
+            parent = d.parent[node].x;
+            __syncwarp(gmask);
+        }
+        __syncwarp(gmask);  // the words are read before the next group's are written
     }
 }
 
@@ -195,13 +276,16 @@ __device__ __forceinline__ F4a mat(const float* m, float x, float y, float z) {
 }
 
 // Per node: covariance, eigen-solve, metrics, screen coverage, score, queue key.
-__global__ void __launch_bounds__(256) k_analyze(Dev d, const RollSum* roll, NodeAnalysis* out,
+__global__ void __launch_bounds__(256) k_analyze(Dev d, RollSum* roll, NodeAnalysis* out,
                                                  float* features, AnalysisParams prm, Frame f,
                                                  AnalysisCounters* ac) {
     const uint32_t nn = d.ctr->numNodes;
     const float cube = fmaxf(fmaxf(f.boxMax[0] - f.boxMin[0], f.boxMax[1] - f.boxMin[1]), f.boxMax[2] - f.boxMin[2]);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
-        const RollSum r = roll[i];
+        // from the root's origin (k_roll) to the node's
+        RollSum r = roll[i];
+        rollRebase<false>(r, d.level[i], d.nodeX[i], d.nodeY[i], d.nodeZ[i]);
+        roll[i] = r;
         NodeAnalysis o;
         o.count = r.n;
         o.lastTouched = r.lastTouched;
@@ -344,7 +428,7 @@ __global__ void __launch_bounds__(256) k_analyze(Dev d, const RollSum* roll, Nod
 // node's surface variation is its partial one plus the network's predicted
 // correction (output 0, x 1/300).
 __global__ void __launch_bounds__(256) k_score(Dev d, NodeAnalysis* out, const float* pred, unsigned long long* keys,
-                                               AnalysisParams prm, AnalysisCounters* ac) {
+                                               uint32_t* hist, AnalysisParams prm, AnalysisCounters* ac) {
     const uint32_t nn = d.ctr->numNodes;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
         NodeAnalysis o = out[i];
@@ -358,56 +442,67 @@ __global__ void __launch_bounds__(256) k_score(Dev d, NodeAnalysis* out, const f
         out[i].score = score;
         const bool eligible = score > 0.0f && (prm.frontierOnly == 0u || (o.flags & kAnalysisFrontier));
         keys[i] = eligible ? (((unsigned long long)__float_as_uint(score) << 32) | (0xFFFFFFFFu - i)) : 0ull;
-        if (eligible) atomicAdd(&ac->eligible, 1u);
-    }
-}
-
-// Radix select of the queue: a 65536-bin histogram of the keys' top 16 bits.
-__global__ void __launch_bounds__(256) k_queue_hist(const Dev d, const unsigned long long* keys, uint32_t* hist) {
-    const uint32_t nn = d.ctr->numNodes;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
-        const unsigned long long k = keys[i];
-        if (k) atomicAdd(&hist[(uint32_t)(k >> 48)], 1u);
-    }
-}
-
-// One block: the lowest bin b such that the bins >= b hold at least K keys.
-__global__ void __launch_bounds__(1024) k_queue_threshold(const uint32_t* hist, uint32_t K, AnalysisCounters* ac) {
-    __shared__ uint32_t s_sum[1024];
-    // each thread owns 64 consecutive bins, counted from the top
-    uint32_t local = 0;
-    const uint32_t t = threadIdx.x;
-    for (uint32_t j = 0; j < 64; j++) local += hist[65535u - (t * 64u + j)];
-    s_sum[t] = local;
-    __syncthreads();
-    if (t == 0) {
-        uint32_t acc = 0;
-        uint32_t thr = 0;
-        bool found = false;
-        for (uint32_t u = 0; u < 1024 && !found; u++) {
-            if (acc + s_sum[u] >= K) {
-                for (uint32_t j = 0; j < 64; j++) {
-                    const uint32_t bin = 65535u - (u * 64u + j);
-                    acc += hist[bin];
-                    if (acc >= K) {
-                        thr = bin;
-                        found = true;
-                        break;
-                    }
-                }
-            } else {
-                acc += s_sum[u];
-            }
+        if (eligible) {
+            atomicAdd(&ac->eligible, 1u);
+            atomicAdd(&hist[__float_as_uint(score) >> 16], 1u);
         }
-        ac->thresholdBin = found ? thr : 0u;
-        ac->numCandidates = 0;
+    }
+}
+
+// Radix select of the queue, over k_score's 65536-bin histogram of the keys'
+// top 16 bits: the lowest bin b such that the bins >= b hold at least K keys.
+// One block; warp w owns 2,048 consecutive bins counted from the top, read as
+// 16 coalesced rows of 16 bytes a lane, all in flight. Only the warp in which
+// the count reaches K looks closer. Bound by one SM reading 256 KB: 77 us with
+// a load per bin and a scan by one thread, 21 us with 16 loads a thread at a
+// stride of 256 B, 5 us so.
+__global__ void __launch_bounds__(1024) k_queue_threshold(const uint32_t* hist, uint32_t K, AnalysisCounters* ac) {
+    __shared__ uint32_t s_warp[32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    // row j, lane l: bins top - 128 j - 4 l - 3 .. top - 128 j - 4 l
+    const uint32_t top = 65535u - warp * 2048u;
+    uint4 v[16];
+#pragma unroll
+    for (uint32_t j = 0; j < 16u; j++)
+        v[j] = __ldcg(reinterpret_cast<const uint4*>(hist + (top - 128u * j - 4u * lane - 3u)));
+    uint32_t local = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < 16u; j++) local += v[j].x + v[j].y + v[j].z + v[j].w;
+    const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, local);
+    if (lane == 0u) s_warp[warp] = sum;
+    __syncthreads();
+    uint32_t above = 0;
+    for (uint32_t w = 0; w < warp; w++) above += s_warp[w];
+    // fewer than K keys: the threshold stays 0, all of them
+    if (above >= K || above + sum < K) return;
+#pragma unroll
+    for (uint32_t j = 0; j < 16u; j++) {
+        const uint32_t row = v[j].x + v[j].y + v[j].z + v[j].w;
+        uint32_t x = row;
+#pragma unroll
+        for (uint32_t o = 1; o < 32u; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= o) x += y;
+        }
+        uint32_t acc = above + x - row;
+        if (acc < K && acc + row >= K) {
+            uint32_t bin = top - 128u * j - 4u * lane;
+            const uint32_t c[4] = {v[j].w, v[j].z, v[j].y, v[j].x};
+            for (uint32_t k = 0; k < 3u && (acc += c[k]) < K; k++) bin--;
+            ac->thresholdBin = bin;
+        }
+        above += __shfl_sync(0xFFFFFFFFu, x, 31);
     }
 }
 
 __global__ void __launch_bounds__(256) k_queue_collect(const Dev d, const unsigned long long* keys,
-                                                       unsigned long long* cand, uint32_t cap, AnalysisCounters* ac) {
+                                                       unsigned long long* cand, uint32_t cap, uint32_t* hist,
+                                                       AnalysisCounters* ac) {
     const uint32_t nn = d.ctr->numNodes;
     const uint32_t thr = ac->thresholdBin;
+    // the histogram back to zero for the next call
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < 65536u / 4u; i += gridDim.x * blockDim.x)
+        reinterpret_cast<uint4*>(hist)[i] = make_uint4(0, 0, 0, 0);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
         const unsigned long long k = keys[i];
         if (k && (uint32_t)(k >> 48) >= thr) {
@@ -466,22 +561,21 @@ __global__ void __launch_bounds__(256) k_refine_set(const uint32_t* queue, const
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < q; i += gridDim.x * blockDim.x) mask[queue[i]] = 1;
 }
 
-void launchRollLevel(const Dev& d, RollSum* roll, uint32_t level, int grid, cudaStream_t s) {
-    k_roll_level<<<grid, 256, 0, s>>>(d, roll, level);
+void launchRoll(const Dev& d, RollSum* roll, uint32_t* rollArrive, AnalysisCounters* ac, int grid, cudaStream_t s) {
+    k_roll<<<grid, kRollThreads, 0, s>>>(d, roll, rollArrive, ac);
 }
-void launchAnalyze(const Dev& d, const RollSum* roll, NodeAnalysis* out, float* features,
+void launchAnalyze(const Dev& d, RollSum* roll, NodeAnalysis* out, float* features,
                    const AnalysisParams& p, const Frame& f, AnalysisCounters* ac, int grid, cudaStream_t s) {
     k_analyze<<<grid, 256, 0, s>>>(d, roll, out, features, p, f, ac);
 }
-void launchScore(const Dev& d, NodeAnalysis* out, const float* predictions, unsigned long long* keys,
+void launchScore(const Dev& d, NodeAnalysis* out, const float* predictions, unsigned long long* keys, uint32_t* hist,
                  const AnalysisParams& p, AnalysisCounters* ac, int grid, cudaStream_t s) {
-    k_score<<<grid, 256, 0, s>>>(d, out, predictions, keys, p, ac);
+    k_score<<<grid, 256, 0, s>>>(d, out, predictions, keys, hist, p, ac);
 }
 void launchQueue(const Dev& d, const unsigned long long* keys, uint32_t* hist, unsigned long long* cand,
                  uint32_t candCap, uint32_t K, uint32_t* queue, AnalysisCounters* ac, int grid, cudaStream_t s) {
-    k_queue_hist<<<grid, 256, 0, s>>>(d, keys, hist);
     k_queue_threshold<<<1, 1024, 0, s>>>(hist, K, ac);
-    k_queue_collect<<<grid, 256, 0, s>>>(d, keys, cand, candCap, ac);
+    k_queue_collect<<<grid, 256, 0, s>>>(d, keys, cand, candCap, hist, ac);
     uint32_t m = 1;
     while (m < candCap) m <<= 1;
     k_queue_sort<<<1, 1024, (size_t)m * 8, s>>>(cand, candCap, K, queue, ac);

@@ -69,11 +69,15 @@ struct AnalysisCounters {
     uint32_t pad[2];
 };
 
-void launchRollLevel(const Dev& d, RollSum* roll, uint32_t level, int grid, cudaStream_t s);
-void launchAnalyze(const Dev& d, const RollSum* roll, NodeAnalysis* out, float* features,
+// Every node's sums from the root's origin (launchAnalyze takes them to the
+// node's), and the counter block zeroed. rollArrive: one counter per
+// sibling group ([maxNodes / 8 + 1]), zero between calls.
+void launchRoll(const Dev& d, RollSum* roll, uint32_t* rollArrive, AnalysisCounters* ac, int grid, cudaStream_t s);
+void launchAnalyze(const Dev& d, RollSum* roll, NodeAnalysis* out, float* features,
                    const AnalysisParams& p, const Frame& f, AnalysisCounters* ac, int grid, cudaStream_t s);
-// Score and queue key per node; predictions (2 per node) are read in kScoreLearned mode.
-void launchScore(const Dev& d, NodeAnalysis* out, const float* predictions, unsigned long long* keys,
+// Score and queue key per node, the keys' top 16 bits counted into hist (65536
+// bins, zero between calls); predictions (2 per node) are read in kScoreLearned mode.
+void launchScore(const Dev& d, NodeAnalysis* out, const float* predictions, unsigned long long* keys, uint32_t* hist,
                  const AnalysisParams& p, AnalysisCounters* ac, int grid, cudaStream_t s);
 void launchQueue(const Dev& d, const unsigned long long* keys, uint32_t* hist, unsigned long long* cand,
                  uint32_t candCap, uint32_t K, uint32_t* queue, AnalysisCounters* ac, int grid, cudaStream_t s);

@@ -36,7 +36,7 @@ static const char* const kKernelNames[K_NUM] = {
     "k_build_begin", "k_batch_begin", "k_count_first", "k_split", "k_spill_copy", "k_recount",
     "k_vox_sample", "k_vox_commit", "k_alloc_points", "k_insert", "k_vox_store", "k_batch_end",
     "k_accumulate", "k_accum_verify", "k_sweep", "k_reset_root", "k_fb_clear", "k_node_flags",
-    "k_frontier", "k_raster", "k_raster_flat", "k_edl", "k_resolve", "k_roll_level", "k_analyze",
+    "k_frontier", "k_raster", "k_raster_flat", "k_edl", "k_resolve", "k_roll", "k_analyze",
     "k_queue", "k_refine", "k_score", "k_mlp_predict", "k_mlp_grad", "k_mlp_adam",
     "k_expand_cond", "k_zero_grids",
     // not a kernel: per-iteration expand passes run inside k_expand_rest
@@ -111,6 +111,7 @@ struct rb_ctx {
     rb::RenderScratch* rs = nullptr;
     // analysis
     rb::RollSum* roll = nullptr;
+    uint32_t* rollArrive = nullptr;
     rb::NodeAnalysis* analysis = nullptr;
     unsigned long long* akeys = nullptr;
     uint32_t* ahist = nullptr;
@@ -615,6 +616,7 @@ rb_status rb_allocate(rb_ctx* c, const rb_cloud_meta* meta, uint64_t budget) {
     ALLOC(c->items, std::max<uint32_t>(cfg.drawlist_capacity, 1), "draw list");
     ALLOC(c->rs, 1, "render scratch");
     ALLOC(c->roll, N, "rolled sums");
+    ALLOC(c->rollArrive, N / 8u + 1u, "roll-up arrivals");
     ALLOC(c->analysis, N, "node analysis");
     ALLOC(c->akeys, N, "queue keys");
     ALLOC(c->ahist, 65536, "queue histogram");
@@ -650,6 +652,8 @@ rb_status rb_allocate(rb_ctx* c, const rb_cloud_meta* meta, uint64_t budget) {
     RB_CUDA(c, cudaMemsetAsync(d.deepCnt, 0, (size_t)rb::kDeepRoots * rb::kDeepCells * 4, c->stream));
     RB_CUDA(c, cudaMemsetAsync(d.deepNode, 0xFF, (size_t)rb::kDeepRoots * rb::kDeepCells * 4, c->stream));
     RB_CUDA(c, cudaMemsetAsync(d.arrive, 0, (size_t)N * 4, c->stream));
+    RB_CUDA(c, cudaMemsetAsync(c->rollArrive, 0, ((size_t)N / 8u + 1u) * 4, c->stream));
+    RB_CUDA(c, cudaMemsetAsync(c->ahist, 0, 65536 * 4, c->stream));
     RB_CUDA(c, cudaMemsetAsync(c->refine.refSlot, 0xFF, (size_t)N * 4, c->stream));
     RB_CUDA(c, cudaMemsetAsync(c->refine.hashKeys, 0xFF, ((size_t)c->refine.hashMask + 1) * 8, c->stream));
     RB_CUDA(c, cudaMallocHost(&c->hostRefine, sizeof(rb::RefineCounters)));
@@ -1188,20 +1192,15 @@ rb_status rb_analyze(rb_ctx* c, const rb_frame* f, const rb_analysis_params* p, 
     if (p->score_mode > RB_SCORE_LEARNED) return fail(c, RB_ERR_INVALID_ARG, "unknown score_mode");
     if (p->score_mode == RB_SCORE_LEARNED && !c->mlpReady)
         return fail(c, RB_ERR_STATE, "learned scoring needs rb_mlp_init or rb_mlp_set_params first");
-    rb_status rst = readCounters(c);
-    if (rst != RB_OK) return rst;
-    const uint32_t numNodes = c->hostCtr->numNodes;
     const rb::Frame fr = toFrame(f);
     RB_CUDA(c, cudaEventRecord(c->evStart, s));
-    RB_CUDA(c, cudaMemsetAsync(c->ahist, 0, 65536 * 4, s));
-    RB_CUDA(c, cudaMemsetAsync(c->actr, 0, sizeof(rb::AnalysisCounters), s));
-    for (int L = rb::kMaxDepth; L >= 0; L--)
-        LAUNCH(c, K_ROLL, 0, rb::launchRollLevel(c->d, c->roll, (uint32_t)L, grid, s));
+    LAUNCH(c, K_ROLL, 0, rb::launchRoll(c->d, c->roll, c->rollArrive, c->actr, grid, s));
     LAUNCH(c, K_ANALYZE, 0, rb::launchAnalyze(c->d, c->roll, c->analysis, c->features, ap, fr, c->actr, grid, s));
     if (p->score_mode == RB_SCORE_LEARNED)
-        LAUNCH(c, K_MLP_PREDICT, numNodes,
-               rb::launchMlpPredict(c->mlp, c->features, numNodes, c->predictions, c->numSMs * 4, s));
-    LAUNCH(c, K_SCORE, 0, rb::launchScore(c->d, c->analysis, c->predictions, c->akeys, ap, c->actr, grid, s));
+        LAUNCH(c, K_MLP_PREDICT, 0,
+               rb::launchMlpPredictCounted(c->mlp, c->features, &c->d.ctr->numNodes, c->predictions, c->numSMs * 2, s));
+    LAUNCH(c, K_SCORE, 0, rb::launchScore(c->d, c->analysis, c->predictions, c->akeys, c->ahist, ap, c->actr, grid,
+                                          s));
     LAUNCH(c, K_QUEUE, 0, rb::launchQueue(c->d, c->akeys, c->ahist, c->acand, kQueueSortCap, p->queue_capacity,
                                           c->aqueue, c->actr, grid, s));
     RB_CUDA(c, cudaGetLastError());

@@ -191,8 +191,10 @@ __device__ __forceinline__ void forwardTile(const SmemWeights& s, const float* _
 }
 
 __global__ void __launch_bounds__(kWarps * 32) k_mlp_predict(const __nv_bfloat16* wq, const float* params,
-                                                             const float* __restrict__ x, uint32_t n, float* y) {
+                                                             const float* __restrict__ x, uint32_t n,
+                                                             const uint32_t* nDev, float* y) {
     __shared__ SmemWeights s;
+    if (nDev) n = *nDev;
     loadWeights(s, wq, params);
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3u;
@@ -462,7 +464,12 @@ __global__ void k_mlp_quantize(const float* params, __nv_bfloat16* wq) {
 void launchMlpPredict(const MlpState& st, const float* x, uint32_t n, float* y, int grid, cudaStream_t s) {
     if (n == 0) return;
     const uint32_t tiles = (n + kBlockSamples - 1) / kBlockSamples;
-    k_mlp_predict<<<tiles < (uint32_t)grid ? (int)tiles : grid, kWarps * 32, 0, s>>>(st.wq, st.params, x, n, y);
+    k_mlp_predict<<<tiles < (uint32_t)grid ? (int)tiles : grid, kWarps * 32, 0, s>>>(st.wq, st.params, x, n, nullptr, y);
+}
+
+void launchMlpPredictCounted(const MlpState& st, const float* x, const uint32_t* nDev, float* y, int grid,
+                             cudaStream_t s) {
+    k_mlp_predict<<<grid, kWarps * 32, 0, s>>>(st.wq, st.params, x, 0u, nDev, y);
 }
 
 constexpr size_t kGradSmem = ((sizeof(SmemWeights) + 15) & ~size_t(15)) + sizeof(SmemStage);

@@ -47,6 +47,9 @@ struct AdamStep {
 };
 
 void launchMlpPredict(const MlpState& st, const float* x, uint32_t n, float* y, int grid, cudaStream_t s);
+// The same over *nDev samples, a count on the device.
+void launchMlpPredictCounted(const MlpState& st, const float* x, const uint32_t* nDev, float* y, int grid,
+                             cudaStream_t s);
 void launchMlpGrad(const MlpState& st, const float* x, const float* t, uint32_t n, int grid, cudaStream_t s);
 void launchMlpAdam(const MlpState& st, const AdamStep& a, cudaStream_t s);
 void launchMlpQuantize(const MlpState& st, cudaStream_t s);

@@ -1,0 +1,67 @@
+"""The one-launch roll-up and the queue's radix select at the trees and queue
+lengths where they could go wrong: a root that never split, one split, deep and
+wide trees, sibling groups that a collapse detached; queues of one entry, of
+every eligible node and of more than there are."""
+import numpy as np
+import pytest
+
+from gpu_helpers import build_gpu, build_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _analyzed(cloud, bmin, bmax, batch, limit, **kw):
+    from remobench_b200.lod import make_frame
+    ctx, _ = build_gpu(cloud, bmin, bmax, batch, max_points_per_node=limit, store_capacity=4 << 30)
+    f = make_frame(bmin, bmax, 1920, 1080, yaw=1.2, pitch=-0.5, radius_scale=0.5)
+    return ctx, f, ctx.analyze(f, frontier_only=False, **kw)
+
+
+@pytest.mark.parametrize("points,limit,nodes", [(700, 1000, 1), (1300, 1000, 9), (60_001, 300, None), (262_144, 2000, None)])
+def test_rollup_equals_the_oracle(c1_cloud, points, limit, nodes):
+    cfg, cloud, bmin, bmax = c1_cloud
+    step = max(1, len(cloud) // points)
+    cloud = np.ascontiguousarray(cloud[::step][:points])
+    ctx, f, _ = _analyzed(cloud, bmin, bmax, 20_011, limit)
+    tree = build_oracle(cloud, bmin, bmax, 20_011, max_points_per_node=limit, persistent_capacity=4 << 30)
+    tree.accumulate((points + 20_010) // 20_011)
+    g = ctx.rollup()
+    assert nodes is None or len(g) == nodes
+    assert np.array_equal(g, tree.rolled_sums()[0])
+    ctx.analyze(f)  # the arrival counters are back at zero
+    assert np.array_equal(ctx.rollup(), g)
+    ctx.close()
+    tree.close()
+
+
+def test_rollup_skips_detached_groups(c1_cloud):
+    cfg, cloud, bmin, bmax = c1_cloud
+    cloud = np.ascontiguousarray(cloud[:200_000])
+    ctx, f, _ = _analyzed(cloud, bmin, bmax, 50_000, 1000)
+    nodes = ctx.nodes()
+    kids = nodes["child"]
+    twigs = [i for i in range(1, len(nodes)) if not nodes["is_leaf"][i] and np.all(nodes["is_leaf"][kids[i]] == 1)]
+    assert ctx.refine_collapse(twigs[::2], max_points=1_000_000).nodes_collapsed == len(twigs[::2])
+    ctx.analyze(f)
+    g = ctx.rollup()
+    assert g[0, 0] == len(cloud)
+    after = ctx.nodes()
+    for i in np.nonzero(after["is_leaf"] == 0)[0]:
+        assert g[i, 0] == g[after["child"][i], 0].sum(), i
+    assert np.all(g[after["is_leaf"] == 1, 0] == after["num_points"][after["is_leaf"] == 1])
+    ctx.close()
+
+
+@pytest.mark.parametrize("k", [1, 2, 31, 1000, 16_384])
+def test_queue_is_the_top_k(c1_cloud, k):
+    cfg, cloud, bmin, bmax = c1_cloud
+    cloud = np.ascontiguousarray(cloud[:400_000])
+    ctx, f, r = _analyzed(cloud, bmin, bmax, 100_000, 1000, queue_capacity=k)
+    for _ in range(2):  # the histogram is back at zero after a call
+        a, q = ctx.analysis(), ctx.queue()
+        ids = np.nonzero(a["score"] > 0)[0]
+        order = ids[np.lexsort((ids, -a["score"][ids]))]
+        assert r.eligible == len(ids) > 1000
+        assert r.overflow == 0 and np.array_equal(q, order[:k])
+        r = ctx.analyze(f, frontier_only=False, queue_capacity=k)
+    ctx.close()
