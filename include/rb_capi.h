@@ -291,7 +291,7 @@ rb_status rb_render(struct rb_ctx* ctx, const rb_frame* frame, uint64_t fb_dev, 
  * they cannot allocate: a frame callback with a hard real-time budget that may
  * not take the allocator's lock or risk an allocation failure mid-frame, or an
  * embedder whose own pool owns all device memory after start-up. It calls no
- * cudaMalloc/cudaFree; its scratch (per-node flags, the draw list, three
+ * cudaMalloc/cudaFree; its scratch (the draw list and its two
  * counters) is a static device array of about 1 MB. rb_allocate resolves the
  * array's device address (cudaGetSymbolAddress, with the context's device
  * current), which under lazy module loading is also when the array is

@@ -27,7 +27,7 @@ using rb::kNone;
 enum KernelId : int {
     K_BUILD_BEGIN, K_BATCH_BEGIN, K_COUNT_FIRST, K_SPLIT, K_SPILL_COPY, K_RECOUNT, K_VOX_SAMPLE,
     K_VOX_COMMIT, K_ALLOC_POINTS, K_INSERT, K_VOX_STORE, K_BATCH_END, K_ACCUMULATE, K_ACCUM_VERIFY,
-    K_SWEEP, K_RESET_ROOT, K_FB_CLEAR, K_NODE_FLAGS, K_FRONTIER, K_RASTER, K_RASTER_FLAT, K_EDL,
+    K_SWEEP, K_RESET_ROOT, K_FB_CLEAR, K_CUT, K_RASTER, K_RASTER_FLAT, K_EDL,
     K_RESOLVE, K_ROLL, K_ANALYZE, K_QUEUE, K_REFINE, K_SCORE, K_MLP_PREDICT, K_MLP_GRAD, K_MLP_ADAM,
     K_EXPAND_COND, K_ZERO_GRIDS, K_EXPAND_PASS, K_DEEP_BOOK, K_DEEP_BIN, K_DEEP_SPLIT, K_DEEP_MOVE,
     K_EXPAND_REST, K_WIREFRAME, K_REFINE_COLORS, K_ALLOC_VOXELS, K_FINISH_LEAVES, K_VOX_LIFT, K_VOX_SAMPLE_LEVELS, K_DEEPEN, K_COLLAPSE, K_NUM
@@ -35,8 +35,7 @@ enum KernelId : int {
 static const char* const kKernelNames[K_NUM] = {
     "k_build_begin", "k_batch_begin", "k_count_first", "k_split", "k_spill_copy", "k_recount",
     "k_vox_sample", "k_vox_commit", "k_alloc_points", "k_insert", "k_vox_store", "k_batch_end",
-    "k_accumulate", "k_accum_verify", "k_sweep", "k_reset_root", "k_fb_clear", "k_node_flags",
-    "k_frontier", "k_raster", "k_raster_flat", "k_edl", "k_resolve", "k_roll", "k_analyze",
+    "k_accumulate", "k_accum_verify", "k_sweep", "k_reset_root", "k_fb_clear", "k_cut", "k_raster", "k_raster_flat", "k_edl", "k_resolve", "k_roll", "k_analyze",
     "k_queue", "k_refine", "k_score", "k_mlp_predict", "k_mlp_grad", "k_mlp_adam",
     "k_expand_cond", "k_zero_grids",
     // not a kernel: per-iteration expand passes run inside k_expand_rest
@@ -103,11 +102,9 @@ struct rb_ctx {
     Counters* hostCtr = nullptr;  // pinned mirror
     rb::SweepStats* hostSweep = nullptr;
     rb::AccumGlobals* hostAccum = nullptr;
-    rb::RenderScratch* hostRs = nullptr;
+    rb::RenderResult* hostRs = nullptr;
     // render scratch
-    uint8_t* vis = nullptr;
-    uint8_t* large = nullptr;
-    uint32_t* items = nullptr;
+    rb::DrawItem* items = nullptr;
     rb::RenderScratch* rs = nullptr;
     // analysis
     rb::RollSum* roll = nullptr;
@@ -436,7 +433,6 @@ void rb_release(rb_ctx* c) {
         c->slotFree[i] = c->slotFull[i] = nullptr;
     }
     c->d = Dev{};
-    c->vis = c->large = nullptr;
     c->items = nullptr;
     c->rs = nullptr;
     c->ingestRing = nullptr;
@@ -485,6 +481,7 @@ rb_status rb_allocate(rb_ctx* c, const rb_cloud_meta* meta, uint64_t budget) {
     d.maxNodes = cfg.max_nodes;
     d.maxPointsPerNode = cfg.max_points_per_node;
     d.ppc = cfg.points_per_chunk;
+    d.ppcRecip = (uint32_t)std::min<uint64_t>((1ull << 32) / d.ppc, 0xFFFFFFFFull);
     d.maxExpandIters = cfg.max_expand_iters;
     d.voxelMode = cfg.voxel_mode;
     d.safetyMargin = cfg.safety_margin;
@@ -498,7 +495,7 @@ rb_status rb_allocate(rb_ctx* c, const rb_cloud_meta* meta, uint64_t budget) {
     if (cfg.pipeline == RB_PIPELINE_FLAT) {
         // flat keeps no tree: render scratch only
         if (devAlloc(c, &c->rs, 1, "render scratch") != RB_OK) return RB_ERR_OUT_OF_MEMORY;
-        RB_CUDA(c, cudaMallocHost(&c->hostRs, sizeof(rb::RenderScratch)));
+        RB_CUDA(c, cudaMallocHost(&c->hostRs, sizeof(rb::RenderResult)));
         RB_CUDA(c, cudaMallocHost(&c->hostCtr, sizeof(Counters)));
         c->allocated = true;
         return RB_OK;
@@ -611,8 +608,6 @@ rb_status rb_allocate(rb_ctx* c, const rb_cloud_meta* meta, uint64_t budget) {
     ALLOC(d.deepPar, N / 8u + 1u, "expand round split lists");
     d.zeroCap = N / 8u + 1u;
     ALLOC(d.zeroList, d.zeroCap, "grids to zero");
-    ALLOC(c->vis, N, "visible flags");
-    ALLOC(c->large, N, "large flags");
     ALLOC(c->items, std::max<uint32_t>(cfg.drawlist_capacity, 1), "draw list");
     ALLOC(c->rs, 1, "render scratch");
     ALLOC(c->roll, N, "rolled sums");
@@ -662,7 +657,7 @@ rb_status rb_allocate(rb_ctx* c, const rb_cloud_meta* meta, uint64_t budget) {
     std::memset(c->hostCtr, 0, sizeof(Counters));
     RB_CUDA(c, cudaMallocHost(&c->hostSweep, sizeof(rb::SweepStats)));
     RB_CUDA(c, cudaMallocHost(&c->hostAccum, sizeof(rb::AccumGlobals)));
-    RB_CUDA(c, cudaMallocHost(&c->hostRs, sizeof(rb::RenderScratch)));
+    RB_CUDA(c, cudaMallocHost(&c->hostRs, sizeof(rb::RenderResult)));
     RB_CUDA(c, cudaMallocHost(&c->hostActr, sizeof(rb::AnalysisCounters)));
     RB_CUDA(c, cudaMallocHost(&c->hostRing, sizeof(rb::RingDesc)));
     std::memset(c->hostRing, 0, sizeof(rb::RingDesc));
@@ -943,9 +938,9 @@ static rb_status finishFrame(rb_ctx* c, const rb_frame* f, unsigned long long* f
     // EDL in place: it reads only its neighbours' depths, which it never
     // writes (a pixel's shading changes its colour half only)
     if (f->enable_edl)
-        LAUNCH(c, K_EDL, npx, rb::launchEdl(fb, fb, (uint32_t)f->width, (uint32_t)f->height, f->edl_strength,
-                                            c->numSMs * 8, c->stream));
-    if (rgba) LAUNCH(c, K_RESOLVE, npx, rb::launchResolve(fb, rgba, npx, c->numSMs * 8, c->stream));
+        LAUNCH(c, K_EDL, npx, rb::launchEdl(fb, rgba, (uint32_t)f->width, (uint32_t)f->height, f->edl_strength,
+                                            c->stream));
+    else if (rgba) LAUNCH(c, K_RESOLVE, npx, rb::launchResolve(fb, rgba, npx, c->numSMs * 8, c->stream));
     return RB_OK;
 }
 
@@ -960,25 +955,20 @@ rb_status rb_render(rb_ctx* c, const rb_frame* f, uint64_t fbDev, uint64_t rgbaD
     const rb::Frame fr = toFrame(f);
     const uint32_t cap = std::max<uint32_t>(c->cfg.drawlist_capacity, 1);
     RB_CUDA(c, cudaEventRecord(c->evStart, c->stream));
-    LAUNCH(c, K_FB_CLEAR, npx, rb::launchFbClear(fb, npx, c->numSMs * 8, c->stream));
-    LAUNCH(c, K_NODE_FLAGS, 0, rb::launchNodeFlags(c->d, fr, c->vis, c->large,
-                                                   reinterpret_cast<const uint8_t*>(forceDev), c->rs,
-                                                   c->numSMs * 4, c->stream));
-    LAUNCH(c, K_FRONTIER, 0, rb::launchFrontier(c->d, c->vis, c->large, c->rs, c->items, cap, c->numSMs * 4,
-                                                c->stream));
-    LAUNCH(c, K_RASTER, 0, rb::launchRaster(c->d, fr, fb, c->rs, c->items, cap, c->numSMs * 8, c->stream));
-    // EDL, then the boxes (remolod_render.cu:183-189), then the resolve
-    rb_status st = finishFrame(c, f, fb, nullptr, npx);
+    LAUNCH(c, K_CUT, npx, rb::launchCut(c->d, fr, fb, npx, reinterpret_cast<const uint8_t*>(forceDev), c->rs, c->items,
+                                        cap, c->numSMs * 8, c->stream));
+    LAUNCH(c, K_RASTER, 0, rb::launchRaster(c->d, fr, fb, c->rs, c->items, cap, c->hostRs, c->numSMs * 8, c->stream));
+    // EDL, then the boxes (remolod_render.cu:183-189), then the resolve: with
+    // EDL's own pass unless boxes come between
+    auto* rgba = reinterpret_cast<uint32_t*>(rgbaDev);
+    rb_status st = finishFrame(c, f, fb, f->show_bounding_box ? nullptr : rgba, npx);
     if (st != RB_OK) return st;
-    if (f->show_bounding_box)
+    if (f->show_bounding_box) {
         LAUNCH(c, K_WIREFRAME, 0, rb::launchWireframe(c->d, fr, fb, c->rs, c->items, cap, c->numSMs * 8, c->stream));
-    if (rgbaDev)
-        LAUNCH(c, K_RESOLVE, npx, rb::launchResolve(fb, reinterpret_cast<uint32_t*>(rgbaDev), npx, c->numSMs * 8,
-                                                    c->stream));
-    if (st != RB_OK) return st;
+        if (rgba) LAUNCH(c, K_RESOLVE, npx, rb::launchResolve(fb, rgba, npx, c->numSMs * 8, c->stream));
+    }
     RB_CUDA(c, cudaGetLastError());
     RB_CUDA(c, cudaEventRecord(c->evStop, c->stream));
-    RB_CUDA(c, cudaMemcpyAsync(c->hostRs, c->rs, sizeof(rb::RenderScratch), cudaMemcpyDeviceToHost, c->stream));
     RB_CUDA(c, cudaStreamSynchronize(c->stream));
     c->lastVisibleNodes = c->hostRs->numItems;
     c->lastVisibleSamples = c->hostRs->samples;
@@ -1006,7 +996,7 @@ rb_status rb_render_flat(rb_ctx* c, const rb_frame* f, uint64_t pointsDev, uint6
     LAUNCH(c, K_FB_CLEAR, npx, rb::launchFbClear(fb, npx, c->numSMs * 8, c->stream));
     if (n)
         LAUNCH(c, K_RASTER_FLAT, n,
-               rb::launchRasterFlat(fr, fb, reinterpret_cast<const rb::Point*>(pointsDev), n, c->numSMs * 16,
+               rb::launchRasterFlat(fr, fb, reinterpret_cast<const rb::Point*>(pointsDev), n, c->numSMs * 8,
                                     c->stream));
     rb_status st = finishFrame(c, f, fb, reinterpret_cast<uint32_t*>(rgbaDev), npx);
     if (st != RB_OK) return st;

@@ -11,7 +11,7 @@ struct rb_ctx;
 
 namespace rb {
 
-struct RenderScratch;
+struct RenderResult;
 
 struct CtxRenderAccess {
     Dev d;                     // the tree (device pointers, capacities)
@@ -22,7 +22,7 @@ struct CtxRenderAccess {
     uint32_t maxNodes;
     uint32_t drawlistCapacity;
     bool allocated;
-    RenderScratch* hostRs;     // pinned, allocated by rb_allocate
+    RenderResult* hostRs;     // pinned, allocated by rb_allocate
     cudaEvent_t evStart, evStop;
 };
 

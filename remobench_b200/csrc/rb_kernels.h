@@ -22,7 +22,26 @@ struct Frame {
     uint32_t showBoundingBox;
 };
 
+// The draw list's cursor and the samples its items hold, points and voxels as
+// counted (rb_render_result). cursor: items emitted in the low kDrawCountBits
+// bits (a node is emitted at most once, and there are at most 2^21), the stored
+// samples of the items so far above them.
 struct RenderScratch {
+    unsigned long long cursor;
+    unsigned long long samples;
+};
+constexpr uint32_t kDrawCountBits = 24;
+constexpr unsigned long long kDrawCountMask = (1ull << kDrawCountBits) - 1ull;
+
+// A draw list entry: the node, and the stored samples of the items before it (a
+// sample takes an arena unit, and there are fewer than 2^32).
+struct DrawItem {
+    uint32_t node;
+    uint32_t first;
+};
+
+// What a render reports, in pinned host memory that k_raster writes.
+struct RenderResult {
     uint32_t numItems;
     uint32_t overflow;
     unsigned long long samples;
@@ -70,19 +89,18 @@ void launchAccumVerify(const Dev& d, int grid, cudaStream_t s);
 
 // Rasterize
 void launchFbClear(unsigned long long* fb, uint64_t npx, int grid, cudaStream_t s);
-void launchNodeFlags(const Dev& d, const Frame& f, uint8_t* vis, uint8_t* large, const uint8_t* force,
-                     RenderScratch* rs, int grid, cudaStream_t s);
-void launchFrontier(const Dev& d, const uint8_t* vis, const uint8_t* large, RenderScratch* rs,
-                    uint32_t* items, uint32_t cap, int grid, cudaStream_t s);
+// The draw list of a frame and its cleared framebuffer.
+void launchCut(const Dev& d, const Frame& f, unsigned long long* fb, uint64_t npx, const uint8_t* force,
+               RenderScratch* rs, DrawItem* items, uint32_t cap, int grid, cudaStream_t s);
 void launchRaster(const Dev& d, const Frame& f, unsigned long long* fb, const RenderScratch* rs,
-                  const uint32_t* items, uint32_t cap, int grid, cudaStream_t s);
+                  const DrawItem* items, uint32_t cap, RenderResult* host, int grid, cudaStream_t s);
 void launchRasterFlat(const Frame& f, unsigned long long* fb, const Point* pts, uint64_t n, int grid,
                       cudaStream_t s);
-void launchEdl(const unsigned long long* src, unsigned long long* dst, uint32_t w, uint32_t h,
-               float strength, int grid, cudaStream_t s);
+// EDL in place; rgba (optional) receives the resolved colours.
+void launchEdl(unsigned long long* fb, uint32_t* rgba, uint32_t w, uint32_t h, float strength, cudaStream_t s);
 void launchResolve(const unsigned long long* fb, uint32_t* rgba, uint64_t npx, int grid, cudaStream_t s);
 // The draw items' bounding boxes as lines (remo_lines.cuh:120-137), after EDL.
 void launchWireframe(const Dev& d, const Frame& f, unsigned long long* fb, const RenderScratch* rs,
-                     const uint32_t* items, uint32_t cap, int grid, cudaStream_t s);
+                     const DrawItem* items, uint32_t cap, int grid, cudaStream_t s);
 
 }  // namespace rb

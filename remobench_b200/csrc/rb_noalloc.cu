@@ -9,8 +9,7 @@
 // per-context scratch that rb_allocate allocates with the tree; this entry
 // point needs none of it.
 //
-// Its scratch -- per-node visible/large flags, the draw list and the three
-// counters -- is one file-scope __device__ array of kScratchBytes (about 1 MB).
+// Its scratch -- the draw list and its two counters -- is one file-scope __device__ array of kScratchBytes (about 1 MB).
 // Host code cannot use the array's name as a device address (on the host it
 // names a host-side stand-in), so rb_allocate, with the context's device
 // current, asks the runtime for the array's device address with
@@ -24,13 +23,11 @@
 // address; a context allocated before a reset must not be used after it.
 //
 // All calls share the array and it keeps the last call's contents: the
-// counters are cleared by the first kernel of every call, and the flags and
-// the draw list are written before they are read. Calls that overlap on the
+// counters are cleared at the start of every call, and the draw list is written
+// before it is read. Calls that overlap on the
 // GPU (two streams, two contexts on one device) race on the array.
 //
-// EDL is applied in place: it changes only the colour half of each pixel and
-// reads only the depth half of its neighbours, so the result equals
-// rb_render's, which shades from a copy.
+// The launches are rb_render's.
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -45,12 +42,10 @@
 
 namespace {
 
-constexpr uint32_t kNoAllocMaxNodes = 262144;  // two flag bytes per node
+constexpr uint32_t kNoAllocMaxNodes = 262144;
 constexpr uint32_t kNoAllocMaxItems = 131072;  // draw list entries (the reference's capacity)
-constexpr size_t kOffVis = 0;
-constexpr size_t kOffLarge = kOffVis + kNoAllocMaxNodes;
-constexpr size_t kOffItems = kOffLarge + kNoAllocMaxNodes;
-constexpr size_t kOffCounters = kOffItems + (size_t)kNoAllocMaxItems * sizeof(uint32_t);
+constexpr size_t kOffItems = 0;
+constexpr size_t kOffCounters = kOffItems + (size_t)kNoAllocMaxItems * sizeof(rb::DrawItem);
 constexpr size_t kScratchBytes = kOffCounters + 256;
 static_assert(kOffItems % 16 == 0 && kOffCounters % 256 == 0, "scratch layout alignment");
 static_assert(sizeof(rb::RenderScratch) <= 256, "counter block must fit its slot");
@@ -103,9 +98,7 @@ namespace {
 // The render itself, with the context's device current.
 rb_status renderNoalloc(rb_ctx* ctx, const rb::CtxRenderAccess& a, unsigned char* base, const rb_frame* f,
                         uint64_t fbDev, uint64_t rgbaDev, uint64_t forceDev, uint32_t cap, rb_render_result* out) {
-    uint8_t* vis = base + kOffVis;
-    uint8_t* large = base + kOffLarge;
-    uint32_t* items = reinterpret_cast<uint32_t*>(base + kOffItems);
+    rb::DrawItem* items = reinterpret_cast<rb::DrawItem*>(base + kOffItems);
     rb::RenderScratch* rs = reinterpret_cast<rb::RenderScratch*>(base + kOffCounters);
 
     const uint64_t npx = (uint64_t)f->width * (uint64_t)f->height;
@@ -127,19 +120,16 @@ rb_status renderNoalloc(rb_ctx* ctx, const rb::CtxRenderAccess& a, unsigned char
     cudaError_t e;
     cudaStream_t s = a.stream;
     if ((e = cudaEventRecord(a.evStart, s)) != cudaSuccess) return cudaFail(ctx, "cudaEventRecord", e);
-    rb::launchFbClear(fb, npx, a.numSMs * 8, s);
-    // the first kernel zeroes the counter block (draw items, overflow, samples)
-    rb::launchNodeFlags(a.d, fr, vis, large, reinterpret_cast<const uint8_t*>(forceDev), rs, a.numSMs * 4, s);
-    rb::launchFrontier(a.d, vis, large, rs, items, cap, a.numSMs * 4, s);
-    rb::launchRaster(a.d, fr, fb, rs, items, cap, a.numSMs * 8, s);
-    if (f->enable_edl) rb::launchEdl(fb, fb, (uint32_t)f->width, (uint32_t)f->height, f->edl_strength,
-                                     a.numSMs * 8, s);
-    if (f->show_bounding_box) rb::launchWireframe(a.d, fr, fb, rs, items, cap, a.numSMs * 8, s);
-    if (rgbaDev) rb::launchResolve(fb, reinterpret_cast<uint32_t*>(rgbaDev), npx, a.numSMs * 8, s);
+    rb::launchCut(a.d, fr, fb, npx, reinterpret_cast<const uint8_t*>(forceDev), rs, items, cap, a.numSMs * 8, s);
+    rb::launchRaster(a.d, fr, fb, rs, items, cap, a.hostRs, a.numSMs * 8, s);
+    auto* rgba = reinterpret_cast<uint32_t*>(rgbaDev);
+    const bool boxes = f->show_bounding_box != 0;
+    if (f->enable_edl) rb::launchEdl(fb, boxes ? nullptr : rgba, (uint32_t)f->width, (uint32_t)f->height,
+                                     f->edl_strength, s);
+    if (boxes) rb::launchWireframe(a.d, fr, fb, rs, items, cap, a.numSMs * 8, s);
+    if (rgba && (boxes || !f->enable_edl)) rb::launchResolve(fb, rgba, npx, a.numSMs * 8, s);
     if ((e = cudaGetLastError()) != cudaSuccess) return cudaFail(ctx, "kernel launch", e);
     if ((e = cudaEventRecord(a.evStop, s)) != cudaSuccess) return cudaFail(ctx, "cudaEventRecord", e);
-    if ((e = cudaMemcpyAsync(a.hostRs, rs, sizeof(rb::RenderScratch), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
-        return cudaFail(ctx, "cudaMemcpyAsync", e);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cudaFail(ctx, "cudaStreamSynchronize", e);
     rb::ctxNoteVisible(ctx, a.hostRs->numItems, a.hostRs->samples);
     if (out) {

@@ -269,6 +269,7 @@ struct Dev {
     uint32_t maxNodes;
     uint32_t maxPointsPerNode;
     uint32_t ppc;            // points per chunk
+    uint32_t ppcRecip;       // floor(2^32 / ppc), 2^32 - 1 for one: quotients at most one low
     uint32_t maxPtChunks;    // chunk queue capacity
     uint32_t arenaUnits;
     uint32_t ptChunkUnits;
