@@ -631,14 +631,15 @@ rb_status rb_allocate(rb_ctx* c, const rb_cloud_meta* meta, uint64_t budget) {
     {
         rb::RefineScratch& r = c->refine;
         r.capacity = cfg.refine_voxel_capacity ? cfg.refine_voxel_capacity : 2097152u;
-        r.hashMask = nextPow2(2ull * r.capacity) - 1u;
+        r.hashMask = std::max<uint32_t>(nextPow2(2ull * r.capacity), 8u) - 1u;
         ALLOC(r.refSlot, N, "refinement node marks");
         ALLOC(r.voxNode, (uint64_t)N + 1, "refinement nodes");
         ALLOC(r.voxBase, (uint64_t)N + 1, "refinement voxel offsets");
         ALLOC(r.acc, r.capacity, "refinement colour sums");
+        ALLOC(r.up, r.capacity, "refinement colour sums from below");
         ALLOC(r.entrySlot, r.capacity, "refinement entry slots");
-        ALLOC(r.hashKeys, (uint64_t)r.hashMask + 1, "refinement cell table keys");
-        ALLOC(r.hashVals, (uint64_t)r.hashMask + 1, "refinement cell table values");
+        ALLOC(r.upSlot, (uint64_t)N + 1, "refinement nodes' next filtered nodes");
+        ALLOC(r.hash, (uint64_t)r.hashMask + 1, "refinement cell table");
         ALLOC(r.ctr, 1, "refinement counters");
     }
 #undef ALLOC
@@ -650,7 +651,7 @@ rb_status rb_allocate(rb_ctx* c, const rb_cloud_meta* meta, uint64_t budget) {
     RB_CUDA(c, cudaMemsetAsync(c->rollArrive, 0, ((size_t)N / 8u + 1u) * 4, c->stream));
     RB_CUDA(c, cudaMemsetAsync(c->ahist, 0, 65536 * 4, c->stream));
     RB_CUDA(c, cudaMemsetAsync(c->refine.refSlot, 0xFF, (size_t)N * 4, c->stream));
-    RB_CUDA(c, cudaMemsetAsync(c->refine.hashKeys, 0xFF, ((size_t)c->refine.hashMask + 1) * 8, c->stream));
+    RB_CUDA(c, cudaMemsetAsync(c->refine.hash, 0xFF, ((size_t)c->refine.hashMask + 1) * 16, c->stream));
     RB_CUDA(c, cudaMallocHost(&c->hostRefine, sizeof(rb::RefineCounters)));
     RB_CUDA(c, cudaMemsetAsync(d.accumGlobals, 0, sizeof(rb::AccumGlobals), c->stream));
     RB_CUDA(c, cudaMallocHost(&c->hostCtr, sizeof(Counters)));

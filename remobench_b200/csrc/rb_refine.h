@@ -12,6 +12,8 @@ struct RefineCounters {
     uint32_t nodes;               // queue prefix filtered
     uint32_t voxels;              // accumulator entries in use
     unsigned long long points;    // (point, filtered ancestor) pairs summed
+    uint32_t units;               // units of points the gathering pass takes
+    uint32_t pad;
 };
 
 // Colour filtering's scratch, sized at allocation: one accumulator entry per
@@ -21,10 +23,11 @@ struct RefineScratch {
     uint32_t* refSlot;            // [maxNodes]
     uint32_t* voxNode;            // [maxNodes + 1] filtered node per slot
     uint32_t* voxBase;            // [maxNodes + 1] first entry per slot, then the total
-    ulonglong4* acc;              // [capacity] r, g, b sums and the count
+    ulonglong4* acc;              // [capacity] r, g, b sums and the count of the points gathered here
+    ulonglong4* up;               // [capacity] the same of the points gathered in filtered nodes below
     uint32_t* entrySlot;          // [capacity] the entry's table slot
-    unsigned long long* hashKeys; // [hashMask + 1], ~0: free
-    uint32_t* hashVals;           // [hashMask + 1]
+    uint2* upSlot;                // [maxNodes + 1] per slot, the next filtered node up that has voxels and its level
+    ulonglong2* hash;             // [hashMask + 1] (key, entry), key ~0: free
     RefineCounters* ctr;
     uint32_t capacity;
     uint32_t hashMask;

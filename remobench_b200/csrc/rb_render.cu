@@ -316,18 +316,6 @@ __device__ __forceinline__ uint32_t itemColor(int32_t mode, uint32_t node, uint3
     return hashColor((unsigned long long)level * 2654435761ull);
 }
 
-// A slot's chunk and its place in it: slot / ppc and slot % ppc through the
-// rounded-down reciprocal (Dev::ppcRecip), whose quotient is at most one low.
-__device__ __forceinline__ uint32_t chunkOf(const Dev& d, uint32_t slot, uint32_t& within) {
-    uint32_t q = __umulhi(slot, d.ppcRecip);
-    within = slot - q * d.ppc;
-    if (within >= d.ppc) {
-        within -= d.ppc;
-        q++;
-    }
-    return q;
-}
-
 __device__ __forceinline__ uint32_t listedItems(const RenderScratch* rs, uint32_t cap) {
     return (uint32_t)min(rs->cursor & kDrawCountMask, (unsigned long long)cap);
 }

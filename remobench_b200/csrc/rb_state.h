@@ -310,6 +310,17 @@ __device__ __forceinline__ uint32_t* chunkIndices(const Dev& d, uint32_t phys) {
 __device__ __forceinline__ uint32_t* gridWordsAt(const Dev& d, uint32_t g) {
     return reinterpret_cast<uint32_t*>(d.arena + (uint64_t)g * 16u);
 }
+// A slot's chunk and its place in it: slot / ppc and slot % ppc through the
+// rounded-down reciprocal (Dev::ppcRecip), whose quotient is at most one low.
+__device__ __forceinline__ uint32_t chunkOf(const Dev& d, uint32_t slot, uint32_t& within) {
+    uint32_t q = __umulhi(slot, d.ppcRecip);
+    within = slot - q * d.ppc;
+    if (within >= d.ppc) {
+        within -= d.ppc;
+        q++;
+    }
+    return q;
+}
 // Bump allocation of `units` 16-byte units; kNone when the arena is full.
 __device__ __forceinline__ uint32_t arenaAlloc(const Dev& d, uint32_t units) {
     const uint32_t off = atomicAdd(&d.ctr->arenaBump, units);

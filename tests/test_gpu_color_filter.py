@@ -1,0 +1,44 @@
+"""Colour filtering where its units, tables and chains could go wrong: chunks of
+one point and longer than a unit, a root that never split, queues of nested
+nodes and of leaves without voxels, points past the declared box, a capacity
+that admits part of the queue."""
+import numpy as np
+import pytest
+
+from gpu_helpers import build_gpu, build_oracle, compare_voxels
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("points,ppc,limit,shrink,capacity", [
+    (900, 1000, 1000, 1.0, 0), (1_100, 1, 1000, 1.0, 0), (50_001, 7, 300, 1.0, 0), (50_001, 5000, 12_000, 1.0, 0),
+    (200_000, 1000, 700, 1.0, 0), (200_000, 1000, 700, 0.8, 0), (200_000, 1000, 5000, 1.0, 20_000)])
+def test_filtered_colours_equal_the_oracle(c1_cloud, points, ppc, limit, shrink, capacity):
+    from remobench_b200.lod import make_frame
+    _, cloud, bmin, bmax = c1_cloud
+    cloud = np.ascontiguousarray(cloud[::len(cloud) // points][:points])
+    bmax = (np.asarray(bmax) * np.float32(shrink)).astype(np.float32)
+    cfg = dict(points_per_chunk=ppc, max_points_per_node=limit)
+    ctx, _ = build_gpu(cloud, bmin, bmax, 20_011, store_capacity=4 << 30, refine_voxel_capacity=capacity, **cfg)
+    tree = build_oracle(cloud, bmin, bmax, 20_011, persistent_capacity=4 << 30, **cfg)
+    f = make_frame(bmin, bmax, 1920, 1080, yaw=1.3, pitch=-0.5, radius_scale=0.5)
+    ctx.analyze(f, min_points=1, frontier_only=False, queue_capacity=16_384)
+    queue = ctx.queue()
+    cap = capacity or 2_097_152
+    for budget in (1, len(queue) // 3, len(queue)):
+        r = ctx.refine_colors(budget)
+        m, nv = tree.refine_colors(queue[:budget], capacity=cap)
+        assert (r.nodes_filtered, r.voxels_filtered) == (m, nv)
+        nodes = ctx.nodes()
+        compare_voxels(ctx, tree, nodes)
+        # every stored point once per filtered node above it (or its own)
+        above = np.zeros(len(nodes), dtype=np.int64)
+        taken = np.zeros(len(nodes), dtype=np.int64)
+        taken[queue[:m]] = 1
+        for i in np.argsort(nodes["level"], kind="stable"):
+            above[i] += taken[i]
+            kids = nodes["child"][i]
+            above[kids[kids >= 0]] += above[i]
+        assert r.points_visited == int((above * nodes["num_points"])[nodes["is_leaf"] == 1].sum())
+    ctx.close()
+    tree.close()
