@@ -122,6 +122,7 @@ struct rb_ctx {
     rb::MlpState mlp{};
     rb::RefineScratch refine{};
     rb::RefineCounters* hostRefine = nullptr;  // pinned
+    float* hostMlp = nullptr;  // pinned: parameters or a gradient on their way out, the loss after them
     bool mlpReady = false;
     uint32_t adamT = 0;
     // device-driven batches: one graph per batch, the ring descriptor it reads
@@ -413,6 +414,8 @@ void rb_release(rb_ctx* c) {
     c->hostActr = nullptr;
     if (c->hostRefine) cudaFreeHost(c->hostRefine);
     c->hostRefine = nullptr;
+    if (c->hostMlp) cudaFreeHost(c->hostMlp);
+    c->hostMlp = nullptr;
     c->refine = rb::RefineScratch{};
     if (c->batchGraph) cudaGraphExecDestroy(c->batchGraph);
     c->batchGraph = nullptr;
@@ -621,11 +624,10 @@ rb_status rb_allocate(rb_ctx* c, const rb_cloud_meta* meta, uint64_t budget) {
     ALLOC(c->features, (uint64_t)N * rb::kIn, "scorer features");
     ALLOC(c->predictions, (uint64_t)N * rb::kOut, "scorer predictions");
     ALLOC(c->mlp.params, rb::kNumParams, "scorer parameters");
-    ALLOC(c->mlp.grad, rb::kNumParams, "scorer gradient");
+    ALLOC(c->mlp.grad, rb::kNumParams + 1, "scorer gradient");
     ALLOC(c->mlp.m, rb::kNumParams, "Adam first moment");
     ALLOC(c->mlp.v, rb::kNumParams, "Adam second moment");
     ALLOC(c->mlp.wq, rb::kNumQuant, "scorer BF16 weights");
-    ALLOC(c->mlp.loss, 1, "scorer loss");
     c->ingestSlots = 3;
     ALLOC(c->ingestRing, (uint64_t)c->ingestSlots * cfg.slot_capacity, "ingest ring");
     {
@@ -648,6 +650,8 @@ rb_status rb_allocate(rb_ctx* c, const rb_cloud_meta* meta, uint64_t budget) {
     RB_CUDA(c, cudaMemsetAsync(d.deepCnt, 0, (size_t)rb::kDeepRoots * rb::kDeepCells * 4, c->stream));
     RB_CUDA(c, cudaMemsetAsync(d.deepNode, 0xFF, (size_t)rb::kDeepRoots * rb::kDeepCells * 4, c->stream));
     RB_CUDA(c, cudaMemsetAsync(d.arrive, 0, (size_t)N * 4, c->stream));
+    RB_CUDA(c, cudaMemsetAsync(c->mlp.grad, 0, sizeof(float) * (rb::kNumParams + 1), c->stream));
+    RB_CUDA(c, cudaMallocHost(&c->hostMlp, sizeof(float) * (rb::kNumParams + 1)));
     RB_CUDA(c, cudaMemsetAsync(c->rollArrive, 0, ((size_t)N / 8u + 1u) * 4, c->stream));
     RB_CUDA(c, cudaMemsetAsync(c->ahist, 0, 65536 * 4, c->stream));
     RB_CUDA(c, cudaMemsetAsync(c->refine.refSlot, 0xFF, (size_t)N * 4, c->stream));
@@ -1297,8 +1301,10 @@ rb_status rb_mlp_get_params(rb_ctx* c, float* params) {
     if (st != RB_OK) return st;
     if (!c->mlpReady) return fail(c, RB_ERR_STATE, "scorer not initialised");
     RB_CUDA(c, cudaSetDevice(c->device));
+    RB_CUDA(c, cudaMemcpyAsync(c->hostMlp, c->mlp.params, sizeof(float) * rb::kNumParams, cudaMemcpyDeviceToHost,
+                               c->stream));
     RB_CUDA(c, cudaStreamSynchronize(c->stream));
-    RB_CUDA(c, cudaMemcpy(params, c->mlp.params, sizeof(float) * rb::kNumParams, cudaMemcpyDeviceToHost));
+    std::memcpy(params, c->hostMlp, sizeof(float) * rb::kNumParams);
     return RB_OK;
 }
 
@@ -1316,9 +1322,7 @@ rb_status rb_mlp_predict(rb_ctx* c, uint64_t x, uint32_t n, uint64_t y) {
 }
 
 static rb_status mlpGrad(rb_ctx* c, uint64_t x, uint64_t t, uint32_t n) {
-    RB_CUDA(c, cudaMemsetAsync(c->mlp.grad, 0, sizeof(float) * rb::kNumParams, c->stream));
-    RB_CUDA(c, cudaMemsetAsync(c->mlp.loss, 0, sizeof(float), c->stream));
-    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((n + 63) / 64, (uint64_t)c->numSMs));
+    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)n + 63) / 64, (uint64_t)c->numSMs * 2));
     LAUNCH(c, K_MLP_GRAD, n, rb::launchMlpGrad(c->mlp, reinterpret_cast<const float*>(x),
                                                reinterpret_cast<const float*>(t), n, grid, c->stream));
     RB_CUDA(c, cudaGetLastError());
@@ -1333,12 +1337,13 @@ rb_status rb_mlp_gradients(rb_ctx* c, uint64_t x, uint64_t t, uint32_t n, float*
     RB_CUDA(c, cudaSetDevice(c->device));
     st = mlpGrad(c, x, t, n);
     if (st != RB_OK) return st;
+    // the gradient and the loss after it in one copy, cleared for the next call
+    RB_CUDA(c, cudaMemcpyAsync(c->hostMlp, c->mlp.grad, sizeof(float) * (rb::kNumParams + 1), cudaMemcpyDeviceToHost,
+                               c->stream));
+    RB_CUDA(c, cudaMemsetAsync(c->mlp.grad, 0, sizeof(float) * (rb::kNumParams + 1), c->stream));
     RB_CUDA(c, cudaStreamSynchronize(c->stream));
-    if (grad) RB_CUDA(c, cudaMemcpy(grad, c->mlp.grad, sizeof(float) * rb::kNumParams, cudaMemcpyDeviceToHost));
-    if (loss) {
-        RB_CUDA(c, cudaMemcpy(loss, c->mlp.loss, sizeof(float), cudaMemcpyDeviceToHost));
-        *loss /= (float)n;
-    }
+    if (grad) std::memcpy(grad, c->hostMlp, sizeof(float) * rb::kNumParams);
+    if (loss) *loss = c->hostMlp[rb::kNumParams] / (float)n;
     return RB_OK;
 }
 
@@ -1358,12 +1363,11 @@ rb_status rb_mlp_train_step(rb_ctx* c, uint64_t x, uint64_t t, uint32_t n, float
     a.eps = 1e-8f;
     a.bc1 = (float)(1.0 - std::pow(0.9, (double)c->adamT));
     a.bc2 = (float)(1.0 - std::pow(0.999, (double)c->adamT));
-    LAUNCH(c, K_MLP_ADAM, 0, rb::launchMlpAdam(c->mlp, a, c->stream));
+    LAUNCH(c, K_MLP_ADAM, 0, rb::launchMlpAdam(c->mlp, a, c->hostMlp + rb::kNumParams, c->stream));
     RB_CUDA(c, cudaGetLastError());
     if (loss) {
-        RB_CUDA(c, cudaMemcpyAsync(loss, c->mlp.loss, sizeof(float), cudaMemcpyDeviceToHost, c->stream));
         RB_CUDA(c, cudaStreamSynchronize(c->stream));
-        *loss /= (float)n;
+        *loss = c->hostMlp[rb::kNumParams] / (float)n;
     }
     return RB_OK;
 }

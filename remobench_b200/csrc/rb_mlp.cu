@@ -16,10 +16,11 @@
 // operand, so activations never leave registers. The backward pass computes
 // dA1 = dZ2 W2 per warp the same way; the weight gradients dW2 = dZ2^T A1 and
 // dW1 = dZ1^T X are contractions over samples, so each block stages its 64
-// samples' dZ2, A1, dZ1 and X transposed in shared memory and each warp
+// samples' dZ2, A1, dZ1 and X in shared memory, sample by sample as the
+// fragments hold them, ldmatrix reads them transposed, and each warp
 // accumulates one 16-row slice of dW2 and dW1 across the block's samples.
-// Bias gradients, the 64 x 2 output layer and its gradient are sums and dot
-// products with 2 outputs: warp shuffles, not GEMMs.
+// Bias gradients, the 64 x 2 output layer and its gradient are FP32 sums and
+// dot products with 2 outputs: kept per lane until the end, not GEMMs.
 //
 // Fragment layouts (PTX ISA, mma.m16n8k16 with .bf16): lane = 4 g + t;
 // A (16 x 16, row-major): {a0, a1, a2, a3} = rows {g, g + 8, g, g + 8}, columns
@@ -48,15 +49,31 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     return *reinterpret_cast<const uint32_t*>(&p);
 }
 
-__device__ __forceinline__ float gelu(float z, float* dgelu) {
+// The forward-only form, as inference has always computed it.
+__device__ __forceinline__ float gelu(float z) {
     const float c = 0.7978845608028654f;
     const float u = c * (z + 0.044715f * z * z * z);
-    const float t = tanhf(u);
-    if (dgelu) {
-        const float du = c * (1.0f + 3.0f * 0.044715f * z * z);
-        *dgelu = 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * du;
-    }
-    return 0.5f * z * (1.0f + t);
+    return 0.5f * z * (1.0f + tanhf(u));
+}
+
+// With its derivative, through (1 + tanh(u)) / 2 = 1 / (1 + e^(-2u)): with
+// p = e^(-2|u|), s = 1 / (1 + p) and r = 1 - s = p s,
+//   gelu(z) = max(z, 0) - |z| r,  gelu'(z) = (z > 0 ? s : r) + 2 z s r u'.
+// No difference of near-equal numbers, so its rms error against FP64 is at or
+// below the tanhf form's (9.3e-9 against 1.8e-8 on [-3, 0), 4.5e-8 against
+// 5.9e-8 on [0, 3); derivative 1.6e-8 against 3.7e-8, 5.7e-8 against 5.2e-8,
+// and 4.5e-8 against 1.9e-7 on [3, 6)), at half the instructions: the two GELUs
+// were most of the gradient kernel's.
+__device__ __forceinline__ float geluGrad(float z, float& dgelu) {
+    const float c = 0.7978845608028654f;
+    const float zz = z * z;
+    const float u = c * (z + 0.044715f * zz * z);
+    const float p = expf(-2.0f * fabsf(u));
+    const float s = __fdividef(1.0f, 1.0f + p);
+    const float r = p * s;
+    const float du = c * (1.0f + 3.0f * 0.044715f * zz);
+    dgelu = (z > 0.0f ? s : r) + 2.0f * z * (s * r) * du;
+    return fmaf(-fabsf(z), r, fmaxf(z, 0.0f));
 }
 
 // D += A B on the tensor cores.
@@ -70,27 +87,36 @@ __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint3
 
 __device__ __forceinline__ uint32_t lds32(const __nv_bfloat16* p) { return *reinterpret_cast<const uint32_t*>(p); }
 
-struct SmemWeights {
+struct __align__(16) SmemWeights {
     __nv_bfloat16 w1[kHidden * kW1Row];   // W1[n][k]
     __nv_bfloat16 w2[kHidden * kW2Row];   // W2[n][k]
-    __nv_bfloat16 w2t[kHidden * kW2Row];  // W2^T[k][n] (backward)
     __nv_bfloat16 w3[8 * kW3Row];         // W3[n][k], rows 2..7 zero
     float b1[kHidden], b2[kHidden], b3[8];
     float w3f[kOut][kHidden];             // W3 as FP32 values of its BF16 copy (backward dot products)
 };
 
+// 16 bytes at a time: the BF16 copies start at multiples of eight elements, and
+// every row here and there is one.
 __device__ void loadWeights(SmemWeights& s, const __nv_bfloat16* wq, const float* params) {
-    for (int i = threadIdx.x; i < kHidden * kIn; i += blockDim.x) s.w1[(i / kIn) * kW1Row + i % kIn] = wq[kQW1 + i];
-    for (int i = threadIdx.x; i < kHidden * kHidden; i += blockDim.x) {
-        const int n = i / kHidden, k = i % kHidden;
-        s.w2[n * kW2Row + k] = wq[kQW2 + i];
-        s.w2t[k * kW2Row + n] = wq[kQW2 + i];
-    }
-    for (int i = threadIdx.x; i < 8 * kHidden; i += blockDim.x) {
-        const int n = i / kHidden, k = i % kHidden;
-        const __nv_bfloat16 w = n < kOut ? wq[kQW3 + n * kHidden + k] : __float2bfloat16_rn(0.0f);
-        s.w3[n * kW3Row + k] = w;
-        if (n < kOut) s.w3f[n][k] = __bfloat162float(w);
+    static_assert(kQW1 % 8 == 0 && kQW2 % 8 == 0 && kQW3 % 8 == 0 && kIn % 8 == 0 && kHidden % 8 == 0 &&
+                      kW1Row % 8 == 0 && kW2Row % 8 == 0 && kW3Row % 8 == 0, "16-byte rows");
+    const uint4* q = reinterpret_cast<const uint4*>(wq);
+    for (int i = threadIdx.x; i < kHidden * kIn / 8; i += blockDim.x)
+        *reinterpret_cast<uint4*>(&s.w1[(i / (kIn / 8)) * kW1Row + i % (kIn / 8) * 8]) = q[kQW1 / 8 + i];
+    for (int i = threadIdx.x; i < kHidden * kHidden / 8; i += blockDim.x)
+        *reinterpret_cast<uint4*>(&s.w2[(i / (kHidden / 8)) * kW2Row + i % (kHidden / 8) * 8]) = q[kQW2 / 8 + i];
+    for (int i = threadIdx.x; i < 8 * kHidden / 8; i += blockDim.x) {
+        const int n = i / (kHidden / 8), k = i % (kHidden / 8) * 8;
+        const uint4 w = n < kOut ? q[kQW3 / 8 + i] : make_uint4(0, 0, 0, 0);
+        *reinterpret_cast<uint4*>(&s.w3[n * kW3Row + k]) = w;
+        if (n < kOut) {
+            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&w);
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                s.w3f[n][k + 2 * e] = __low2float(h[e]);
+                s.w3f[n][k + 2 * e + 1] = __high2float(h[e]);
+            }
+        }
     }
     for (int i = threadIdx.x; i < kHidden; i += blockDim.x) {
         s.b1[i] = params[kPB1 + i];
@@ -145,7 +171,7 @@ __device__ __forceinline__ void forwardTile(const SmemWeights& s, const float* _
 #pragma unroll
     for (int i = 0; i < 8; i++)
 #pragma unroll
-        for (int e = 0; e < 4; e++) c[i][e] = gelu(c[i][e], kGrad ? &f.dg1[i][e] : nullptr);
+        for (int e = 0; e < 4; e++) c[i][e] = kGrad ? geluGrad(c[i][e], f.dg1[i][e]) : gelu(c[i][e]);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         f.a1[j][0] = pack2(c[2 * j][0], c[2 * j][1]);
@@ -170,7 +196,7 @@ __device__ __forceinline__ void forwardTile(const SmemWeights& s, const float* _
 #pragma unroll
     for (int i = 0; i < 8; i++)
 #pragma unroll
-        for (int e = 0; e < 4; e++) c[i][e] = gelu(c[i][e], kGrad ? &f.dg2[i][e] : nullptr);
+        for (int e = 0; e < 4; e++) c[i][e] = kGrad ? geluGrad(c[i][e], f.dg2[i][e]) : gelu(c[i][e]);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         f.a2[j][0] = pack2(c[2 * j][0], c[2 * j][1]);
@@ -209,15 +235,33 @@ __global__ void __launch_bounds__(kWarps * 32) k_mlp_predict(const __nv_bfloat16
     }
 }
 
-// The block's staged transposes for the weight-gradient GEMMs: per neuron (or
-// input), its value for each of the block's 64 samples.
-struct SmemStage {
-    __nv_bfloat16 dz2t[kHidden * kSRow];  // dZ2^T [layer-2 neuron][sample]
-    __nv_bfloat16 a1t[kHidden * kSRow];   // A1^T  [layer-1 neuron][sample]
-    __nv_bfloat16 dz1t[kHidden * kSRow];  // dZ1^T [layer-1 neuron][sample]
-    __nv_bfloat16 xt[kIn * kSRow];        // X^T   [input][sample]
-    float red[kOut * kHidden + kHidden + kHidden + 8];  // dW3, db2, db1, db3 block sums
+// The block's values for the weight-gradient GEMMs, per sample.
+struct __align__(16) SmemStage {
+    __nv_bfloat16 dz2[kBlockSamples * kSRow];  // dZ2 [sample][layer-2 neuron]
+    __nv_bfloat16 a1[kBlockSamples * kSRow];   // A1  [sample][layer-1 neuron]
+    __nv_bfloat16 dz1[kBlockSamples * kSRow];  // dZ1 [sample][layer-1 neuron]
+    __nv_bfloat16 x[kBlockSamples * kW1Row];   // X   [sample][input]
 };
+
+// Fragments of stored matrices read transposed. A (16 x 16) from rows that are
+// A's columns: matrices (rows 0-7, cols 0-7), (8-15, 0-7), (0-7, 8-15), (8-15,
+// 8-15) of A, i.e. of the stored matrix its transposes. B (16 x 8) from rows
+// that are B's rows.
+__device__ __forceinline__ void ldmatrixA(uint32_t (&a)[4], const __nv_bfloat16* rows, int stride, int col) {
+    const uint32_t lane = threadIdx.x & 31u, m = lane >> 3, r = lane & 7u;
+    const uint32_t p = (uint32_t)__cvta_generic_to_shared(rows + (r + (m >> 1) * 8) * stride + col + (m & 1) * 8);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(p) : "memory");
+}
+// Two neighbouring B tiles (columns col .. col + 15) over 16 rows.
+__device__ __forceinline__ void ldmatrixB2(uint32_t (&b)[4], const __nv_bfloat16* rows, int stride, int col) {
+    const uint32_t lane = threadIdx.x & 31u, m = lane >> 3, r = lane & 7u;
+    const uint32_t p = (uint32_t)__cvta_generic_to_shared(rows + (r + (m & 1) * 8) * stride + col + (m >> 1) * 8);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]) : "r"(p) : "memory");
+}
+
+__device__ __forceinline__ void sts32(__nv_bfloat16* p, uint32_t v) { *reinterpret_cast<uint32_t*>(p) = v; }
 
 // Sum of v over the 8 row groups of a fragment (lanes with equal t).
 __device__ __forceinline__ float sumRows(float v) {
@@ -227,40 +271,52 @@ __device__ __forceinline__ float sumRows(float v) {
     return v;
 }
 
-// Gradient of the mean loss over n samples, added into grad (kNumParams
-// floats, zeroed by the caller); loss sum added into lossSum.
-__global__ void __launch_bounds__(kWarps * 32) k_mlp_grad(const __nv_bfloat16* wq, const float* params,
-                                                          const float* __restrict__ x, const float* __restrict__ tgt,
-                                                          uint32_t n, float* grad, float* lossSum) {
-    // 55 KB: over the static limit, so dynamic
+// Gradient of the mean loss over n samples, added into grad (kNumParams floats
+// and the loss sum after them, zero before the launch).
+//
+// Bound by instruction issue, half of it the 128 GELUs of a sample with their
+// derivatives; the tensor cores idle (12.6 GFLOP at 400k samples, 8 us of their
+// peak). At 400,003 samples: 463 us with tanhf, transposes staged two bytes at a
+// time, the FP32 sums reduced by shuffles in every tile and one block per SM;
+// 127 us so, at two (141 at three, which spill). At 2,048 samples 16.1 and 9.9 us.
+__global__ void __launch_bounds__(kWarps * 32, 2) k_mlp_grad(const __nv_bfloat16* wq, const float* params,
+                                                             const float* __restrict__ x,
+                                                             const float* __restrict__ tgt, uint32_t n, float* grad) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     SmemWeights& s = *reinterpret_cast<SmemWeights*>(s_raw);
-    SmemStage& st = *reinterpret_cast<SmemStage*>(s_raw + ((sizeof(SmemWeights) + 15) & ~size_t(15)));
+    SmemStage& st = *reinterpret_cast<SmemStage*>(s_raw + sizeof(SmemWeights));
     loadWeights(s, wq, params);
-    for (int i = threadIdx.x; i < (int)(sizeof(st.red) / sizeof(float)); i += blockDim.x) st.red[i] = 0.0f;
     __syncthreads();
-    float* sdw3 = st.red;
-    float* sdb2 = st.red + kOut * kHidden;
-    float* sdb1 = sdb2 + kHidden;
-    float* sdb3 = sdb1 + kHidden;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3u;
     const float invN = 1.0f / (float)n;
     // this warp's slices of the weight gradients: rows 16 warp .. +15 of dW2 (8 column tiles) and dW1 (2)
     float dw2[8][4], dw1[2][4];
+    // this lane's FP32 sums over its rows g, g + 8 of every tile: per column pair
+    // (8 i + 2 t, + 1) db2, db1 and dW3's two rows; db3 and the loss on lanes t == 0
+    float db2[8][2], db1[8][2], dw3[2][8][2], db3[2] = {0.0f, 0.0f}, loss = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 8; i++)
+    for (int i = 0; i < 8; i++) {
 #pragma unroll
         for (int e = 0; e < 4; e++) dw2[i][e] = 0.0f;
+#pragma unroll
+        for (int e = 0; e < 2; e++) db2[i][e] = db1[i][e] = dw3[0][i][e] = dw3[1][i][e] = 0.0f;
+    }
 #pragma unroll
     for (int i = 0; i < 2; i++)
 #pragma unroll
         for (int e = 0; e < 4; e++) dw1[i][e] = 0.0f;
-    float loss = 0.0f;
     for (uint32_t block0 = blockIdx.x * kBlockSamples; block0 < n; block0 += gridDim.x * kBlockSamples) {
         const uint32_t base = block0 + warp * kTile;
-        const uint32_t col0 = warp * kTile;  // this warp's sample columns in the staged transposes
+        const uint32_t row0 = warp * kTile + g;  // this lane's first staged sample; the other is row0 + 8
         Fwd f;
         forwardTile<true>(s, x, n, base, f);
+        // A1 and X as they are
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) sts32(&st.a1[(row0 + 8 * (q & 1)) * kSRow + 16 * j + 2 * t + 8 * (q >> 1)], f.a1[j][q]);
+#pragma unroll
+        for (int q = 0; q < 4; q++) sts32(&st.x[(row0 + 8 * (q & 1)) * kW1Row + 2 * t + 8 * (q >> 1)], f.xa[q]);
         // the loss and dY per sample (lanes t == 0 hold the outputs of rows g and g + 8)
         float dy[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
         if (t == 0) {
@@ -277,143 +333,85 @@ __global__ void __launch_bounds__(kWarps * 32) k_mlp_grad(const __nv_bfloat16* w
                 dy[h][0] = 2.0f * e * invN;
                 dy[h][1] = (sig - tv.y) * invN;
             }
+            db3[0] += dy[0][0] + dy[1][0];
+            db3[1] += dy[0][1] + dy[1][1];
         }
 #pragma unroll
         for (int h = 0; h < 2; h++)
 #pragma unroll
             for (int o = 0; o < 2; o++) dy[h][o] = __shfl_sync(0xFFFFFFFFu, dy[h][o], lane & ~3u);
-        {
-            // db3: every lane of a row group holds its rows' dY; count it once (t == 0)
-            const float s0 = sumRows(t == 0 ? dy[0][0] + dy[1][0] : 0.0f);
-            const float s1 = sumRows(t == 0 ? dy[0][1] + dy[1][1] : 0.0f);
-            if (lane == 0) {
-                atomicAdd(&sdb3[0], s0);
-                atomicAdd(&sdb3[1], s1);
-            }
-        }
-        // layer 3 backward: dW3 += dY^T A2, dA2 = dY W3, dZ2 = dA2 gelu'(Z2)
-        float dz2[8][4];
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const int col = 8 * i + 2 * t + (e & 1);
-                const int h = e >> 1;
-                dz2[i][e] = (dy[h][0] * s.w3f[0][col] + dy[h][1] * s.w3f[1][col]) * f.dg2[i][e];
-            }
-            // A2 values of this tile (BF16 as stored in the fragments)
-            const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&f.a2[i >> 1][(i & 1) * 2]);
-            const __nv_bfloat162 hi = *reinterpret_cast<const __nv_bfloat162*>(&f.a2[i >> 1][(i & 1) * 2 + 1]);
-            const float a2v[4] = {__low2float(lo), __high2float(lo), __low2float(hi), __high2float(hi)};
-#pragma unroll
-            for (int o = 0; o < 2; o++) {
-                float w0 = dy[0][o] * a2v[0] + dy[1][o] * a2v[2];
-                float w1 = dy[0][o] * a2v[1] + dy[1][o] * a2v[3];
-                w0 = sumRows(w0);
-                w1 = sumRows(w1);
-                if (g == 0) {
-                    atomicAdd(&sdw3[o * kHidden + 8 * i + 2 * t], w0);
-                    atomicAdd(&sdw3[o * kHidden + 8 * i + 2 * t + 1], w1);
-                }
-            }
-            float b0 = sumRows(dz2[i][0] + dz2[i][2]), b1 = sumRows(dz2[i][1] + dz2[i][3]);
-            if (g == 0) {
-                atomicAdd(&sdb2[8 * i + 2 * t], b0);
-                atomicAdd(&sdb2[8 * i + 2 * t + 1], b1);
-            }
-        }
-        // dZ2 as the A operand of dA1 = dZ2 W2 (K = layer-2 neurons), and staged transposed
+        // layer 3 backward: dW3 += dY^T A2, dA2 = dY W3, dZ2 = dA2 gelu'(Z2);
+        // dZ2 rounded to BF16 is the A operand of dA1 = dZ2 W2, and staged
         uint32_t dza[4][4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            dza[j][0] = pack2(dz2[2 * j][0], dz2[2 * j][1]);
-            dza[j][1] = pack2(dz2[2 * j][2], dz2[2 * j][3]);
-            dza[j][2] = pack2(dz2[2 * j + 1][0], dz2[2 * j + 1][1]);
-            dza[j][3] = pack2(dz2[2 * j + 1][2], dz2[2 * j + 1][3]);
-        }
-#pragma unroll
-        for (int i = 0; i < 8; i++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const int col = 8 * i + 2 * t + (e & 1);
-                const int row = g + 8 * (e >> 1);
-                st.dz2t[col * kSRow + col0 + row] = __float2bfloat16_rn(dz2[i][e]);
-            }
-        // A1 and X staged transposed (their BF16 values)
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(&f.a1[j][q]);
-                const int col = 16 * j + 2 * t + 8 * (q >> 1);
-                const int row = g + 8 * (q & 1);
-                st.a1t[col * kSRow + col0 + row] = v.x;
-                st.a1t[(col + 1) * kSRow + col0 + row] = v.y;
-            }
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(&f.xa[q]);
-            const int col = 2 * t + 8 * (q >> 1);
-            const int row = g + 8 * (q & 1);
-            st.xt[col * kSRow + col0 + row] = v.x;
-            st.xt[(col + 1) * kSRow + col0 + row] = v.y;
-        }
-        // layer 2 backward: dA1 = dZ2 W2, dZ1 = dA1 gelu'(Z1)
-#pragma unroll
         for (int i = 0; i < 8; i++) {
-            float c[4] = {0.f, 0.f, 0.f, 0.f};
+            const float2 w0 = *reinterpret_cast<const float2*>(&s.w3f[0][8 * i + 2 * t]);
+            const float2 w1 = *reinterpret_cast<const float2*>(&s.w3f[1][8 * i + 2 * t]);
+            float dz2[4];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                dz2[2 * h] = (dy[h][0] * w0.x + dy[h][1] * w1.x) * f.dg2[i][2 * h];
+                dz2[2 * h + 1] = (dy[h][0] * w0.y + dy[h][1] * w1.y) * f.dg2[i][2 * h + 1];
+                // A2's values of this row (BF16 as stored in the fragments)
+                const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(&f.a2[i >> 1][(i & 1) * 2 + h]);
+                const float vx = __low2float(v), vy = __high2float(v);
+#pragma unroll
+                for (int o = 0; o < 2; o++) {
+                    dw3[o][i][0] += dy[h][o] * vx;
+                    dw3[o][i][1] += dy[h][o] * vy;
+                }
+                db2[i][0] += dz2[2 * h];
+                db2[i][1] += dz2[2 * h + 1];
+                const uint32_t packed = pack2(dz2[2 * h], dz2[2 * h + 1]);
+                dza[i >> 1][(i & 1) * 2 + h] = packed;
+                sts32(&st.dz2[(row0 + 8 * h) * kSRow + 8 * i + 2 * t], packed);
+            }
+        }
+        // layer 2 backward: dA1 = dZ2 W2 (W2's rows are the contraction's), dZ1 = dA1 gelu'(Z1)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            float c[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                // B[k][n] = W2[k][n]: k = layer-2 neuron, n = layer-1 neuron
-                const __nv_bfloat16* w = s.w2t + (8 * i + g) * kW2Row + 16 * j + 2 * t;
-                mma(c, dza[j], lds32(w), lds32(w + 8));
+                uint32_t b[4];
+                ldmatrixB2(b, s.w2 + 16 * j * kW2Row, kW2Row, 16 * i);
+                mma(c[0], dza[j], b[0], b[1]);
+                mma(c[1], dza[j], b[2], b[3]);
             }
-            float dz1[4];
 #pragma unroll
-            for (int e = 0; e < 4; e++) dz1[e] = c[e] * f.dg1[i][e];
+            for (int u = 0; u < 2; u++) {
+                const int k = 2 * i + u;
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const int col = 8 * i + 2 * t + (e & 1);
-                const int row = g + 8 * (e >> 1);
-                st.dz1t[col * kSRow + col0 + row] = __float2bfloat16_rn(dz1[e]);
-            }
-            float b0 = sumRows(dz1[0] + dz1[2]), b1 = sumRows(dz1[1] + dz1[3]);
-            if (g == 0) {
-                atomicAdd(&sdb1[8 * i + 2 * t], b0);
-                atomicAdd(&sdb1[8 * i + 2 * t + 1], b1);
+                for (int h = 0; h < 2; h++) {
+                    const float d0 = c[u][2 * h] * f.dg1[k][2 * h], d1 = c[u][2 * h + 1] * f.dg1[k][2 * h + 1];
+                    db1[k][0] += d0;
+                    db1[k][1] += d1;
+                    sts32(&st.dz1[(row0 + 8 * h) * kSRow + 8 * k + 2 * t], pack2(d0, d1));
+                }
             }
         }
         __syncthreads();
         // the weight gradients over the block's 64 samples: this warp's 16 rows
-        const int m0 = 16 * warp;
+        const int m0 = 16 * (int)warp;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            uint32_t a[4];
-            const __nv_bfloat16* p = st.dz2t + (m0 + g) * kSRow + 16 * k + 2 * t;
-            a[0] = lds32(p);
-            a[1] = lds32(p + 8 * kSRow);
-            a[2] = lds32(p + 8);
-            a[3] = lds32(p + 8 * kSRow + 8);
+            uint32_t a[4], b[4];
+            ldmatrixA(a, st.dz2 + 16 * k * kSRow, kSRow, m0);
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const __nv_bfloat16* b = st.a1t + (8 * i + g) * kSRow + 16 * k + 2 * t;
-                mma(dw2[i], a, lds32(b), lds32(b + 8));
+            for (int i = 0; i < 4; i++) {
+                ldmatrixB2(b, st.a1 + 16 * k * kSRow, kSRow, 16 * i);
+                mma(dw2[2 * i], a, b[0], b[1]);
+                mma(dw2[2 * i + 1], a, b[2], b[3]);
             }
-            const __nv_bfloat16* q = st.dz1t + (m0 + g) * kSRow + 16 * k + 2 * t;
-            a[0] = lds32(q);
-            a[1] = lds32(q + 8 * kSRow);
-            a[2] = lds32(q + 8);
-            a[3] = lds32(q + 8 * kSRow + 8);
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const __nv_bfloat16* b = st.xt + (8 * i + g) * kSRow + 16 * k + 2 * t;
-                mma(dw1[i], a, lds32(b), lds32(b + 8));
-            }
+            ldmatrixA(a, st.dz1 + 16 * k * kSRow, kSRow, m0);
+            ldmatrixB2(b, st.x + 16 * k * kW1Row, kW1Row, 0);
+            mma(dw1[0], a, b[0], b[1]);
+            mma(dw1[1], a, b[2], b[3]);
         }
         __syncthreads();
     }
-    // this warp's slices of dW2 and dW1, and the block's shuffled sums, into the global gradient
-    const int m0 = 16 * warp;
+    // this warp's slices of dW2 and dW1 into the global gradient
+    const int m0 = 16 * (int)warp;
 #pragma unroll
     for (int i = 0; i < 8; i++)
 #pragma unroll
@@ -428,20 +426,53 @@ __global__ void __launch_bounds__(kWarps * 32) k_mlp_grad(const __nv_bfloat16* w
             const int row = m0 + g + 8 * (e >> 1), col = 8 * i + 2 * t + (e & 1);
             atomicAdd(&grad[kPW1 + row * kIn + col], dw1[i][e]);
         }
-    for (int off = 16; off > 0; off >>= 1) loss += __shfl_xor_sync(0xFFFFFFFFu, loss, off);
-    if (lane == 0) atomicAdd(lossSum, loss);
-    __syncthreads();
-    for (int i = threadIdx.x; i < kOut * kHidden; i += blockDim.x) atomicAdd(&grad[kPW3 + i], sdw3[i]);
-    for (int i = threadIdx.x; i < kHidden; i += blockDim.x) {
-        atomicAdd(&grad[kPB2 + i], sdb2[i]);
-        atomicAdd(&grad[kPB1 + i], sdb1[i]);
+    // the FP32 sums: over the lanes of equal t by shuffles, over the warps in
+    // shared memory (the staging is done with), one atomic per block and entry
+    float* red = reinterpret_cast<float*>(&st);  // [warp][dW3 | db2 | db1 | db3, loss]
+    constexpr int kRed = kOut * kHidden + 2 * kHidden + kOut + 1;
+    static_assert(sizeof(SmemStage) >= kWarps * kRed * sizeof(float), "reduction scratch");
+    float* mine = red + warp * kRed;
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int col = 8 * i + 2 * t + e;
+            const float w30 = sumRows(dw3[0][i][e]), w31 = sumRows(dw3[1][i][e]);
+            const float s2 = sumRows(db2[i][e]), s1 = sumRows(db1[i][e]);
+            if (g == 0) {
+                mine[col] = w30;
+                mine[kHidden + col] = w31;
+                mine[kOut * kHidden + col] = s2;
+                mine[(kOut + 1) * kHidden + col] = s1;
+            }
+        }
+    const float s30 = sumRows(db3[0]), s31 = sumRows(db3[1]), sl = sumRows(loss);
+    if (lane == 0) {
+        mine[kRed - 3] = s30;
+        mine[kRed - 2] = s31;
+        mine[kRed - 1] = sl;
     }
-    if (threadIdx.x < kOut) atomicAdd(&grad[kPB3 + threadIdx.x], sdb3[threadIdx.x]);
+    __syncthreads();
+    for (int i = threadIdx.x; i < kRed; i += blockDim.x) {
+        float v = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kWarps; w++) v += red[w * kRed + i];
+        int to;
+        if (i < kOut * kHidden) to = kPW3 + i;
+        else if (i < (kOut + 1) * kHidden) to = kPB2 + i - kOut * kHidden;
+        else if (i < (kOut + 2) * kHidden) to = kPB1 + i - (kOut + 1) * kHidden;
+        else to = kPB3 + i - (kOut + 2) * kHidden;  // b3, then the loss at kNumParams
+        atomicAdd(&grad[to], v);
+    }
 }
 
-__global__ void k_mlp_adam(float* params, const float* grad, float* m, float* v, __nv_bfloat16* wq, AdamStep a) {
+// One Adam step; leaves the gradient and the loss sum at zero for the next one
+// and the sum in hostLoss (pinned).
+__global__ void k_mlp_adam(float* params, float* grad, float* m, float* v, __nv_bfloat16* wq, AdamStep a,
+                           float* hostLoss) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kNumParams; i += gridDim.x * blockDim.x) {
         const float g = grad[i];
+        grad[i] = 0.0f;
         const float mi = a.beta1 * m[i] + (1.0f - a.beta1) * g;
         const float vi = a.beta2 * v[i] + (1.0f - a.beta2) * g * g;
         m[i] = mi;
@@ -451,6 +482,10 @@ __global__ void k_mlp_adam(float* params, const float* grad, float* m, float* v,
         params[i] = w;
         const int q = quantIndex(i);
         if (q >= 0) wq[q] = __float2bfloat16_rn(w);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *hostLoss = grad[kNumParams];
+        grad[kNumParams] = 0.0f;
     }
 }
 
@@ -472,7 +507,7 @@ void launchMlpPredictCounted(const MlpState& st, const float* x, const uint32_t*
     k_mlp_predict<<<grid, kWarps * 32, 0, s>>>(st.wq, st.params, x, 0u, nDev, y);
 }
 
-constexpr size_t kGradSmem = ((sizeof(SmemWeights) + 15) & ~size_t(15)) + sizeof(SmemStage);
+constexpr size_t kGradSmem = sizeof(SmemWeights) + sizeof(SmemStage);
 
 cudaError_t configureMlp() {
     return cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGradSmem);
@@ -482,11 +517,11 @@ void launchMlpGrad(const MlpState& st, const float* x, const float* t, uint32_t 
     if (n == 0) return;
     const uint32_t tiles = (n + kBlockSamples - 1) / kBlockSamples;
     k_mlp_grad<<<tiles < (uint32_t)grid ? (int)tiles : grid, kWarps * 32, kGradSmem, s>>>(st.wq, st.params, x, t, n,
-                                                                                           st.grad, st.loss);
+                                                                                           st.grad);
 }
 
-void launchMlpAdam(const MlpState& st, const AdamStep& a, cudaStream_t s) {
-    k_mlp_adam<<<(kNumParams + 255) / 256, 256, 0, s>>>(st.params, st.grad, st.m, st.v, st.wq, a);
+void launchMlpAdam(const MlpState& st, const AdamStep& a, float* hostLoss, cudaStream_t s) {
+    k_mlp_adam<<<(kNumParams + 255) / 256, 256, 0, s>>>(st.params, st.grad, st.m, st.v, st.wq, a, hostLoss);
 }
 
 void launchMlpQuantize(const MlpState& st, cudaStream_t s) {

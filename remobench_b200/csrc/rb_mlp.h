@@ -34,11 +34,10 @@ __host__ __device__ inline int quantIndex(int i) {
 
 struct MlpState {
     float* params;       // [kNumParams] FP32 master
-    float* grad;         // [kNumParams]
+    float* grad;         // [kNumParams + 1] gradient, then the summed per-sample loss; zero between calls
     float* m;            // Adam first moment
     float* v;            // Adam second moment
     __nv_bfloat16* wq;   // [kNumQuant]
-    float* loss;         // [1] summed per-sample loss of the last gradient
 };
 
 struct AdamStep {
@@ -51,7 +50,8 @@ void launchMlpPredict(const MlpState& st, const float* x, uint32_t n, float* y, 
 void launchMlpPredictCounted(const MlpState& st, const float* x, const uint32_t* nDev, float* y, int grid,
                              cudaStream_t s);
 void launchMlpGrad(const MlpState& st, const float* x, const float* t, uint32_t n, int grid, cudaStream_t s);
-void launchMlpAdam(const MlpState& st, const AdamStep& a, cudaStream_t s);
+// Clears the gradient it consumes; the loss sum goes to hostLoss (pinned memory).
+void launchMlpAdam(const MlpState& st, const AdamStep& a, float* hostLoss, cudaStream_t s);
 void launchMlpQuantize(const MlpState& st, cudaStream_t s);
 cudaError_t configureMlp();
 
