@@ -1558,13 +1558,23 @@ __global__ void __launch_bounds__(1024, 1) k_expand_rest(Dev d) {
     finishLeavesBody(d, nullptr, 0u);
 }
 
+// A cell's home slot in the batch's table. The 2 x 2 x 2 cells of a brick share
+// one 128-byte line (eight 16-byte slots) and are hashed together, so a warp's
+// neighbouring points and a new cell's siblings meet in few lines; the place
+// within the line is mixed with the brick's hash so that flat surfaces, which
+// fill half of a brick, still spread over all eight. Probing goes from line to
+// line at the same place (nextSlot), so a place's chain is as long as in a table
+// of an eighth of the size at the same load.
 __device__ __forceinline__ uint32_t hashSlot(unsigned long long key, uint32_t mask) {
-    unsigned long long h = key * 0x9E3779B97F4A7C15ull;
+    const uint32_t cell = (uint32_t)key & 0x1FFFFFu;
+    const uint32_t place = (cell & 1u) | ((cell >> 6) & 2u) | ((cell >> 12) & 4u);
+    unsigned long long h = (key & ~0x4081ull) * 0x9E3779B97F4A7C15ull;
     h ^= h >> 29;
     h *= 0xBF58476D1CE4E5B9ull;
     h ^= h >> 32;
-    return (uint32_t)h & mask;
+    return (((uint32_t)h & ~7u) | (((uint32_t)h ^ place) & 7u)) & mask;
 }
+__device__ __forceinline__ uint32_t nextSlot(uint32_t slot, uint32_t mask) { return (slot + 8u) & mask; }
 
 // Records a claimed table slot in the batch's list of new cells.
 __device__ __forceinline__ void listNewCell(const Dev& d, uint32_t e, uint32_t slot) {
@@ -1599,7 +1609,7 @@ __device__ void hashInsertFrom(const Dev& d, unsigned long long key, unsigned lo
             else atomicCAS(vs, kHashEmpty, val);
             return;
         }
-        slot = (slot + 1u) & d.hashMask;
+        slot = nextSlot(slot, d.hashMask);
     }
     atomicOr(&d.ctr->overflowFlags, (uint32_t)kOvfBacklog);
     d.ctr->hashNeedsClear = 1u;
@@ -1617,8 +1627,10 @@ __device__ __forceinline__ uint32_t cellAt(uint32_t x28, uint32_t y28, uint32_t 
 // the tag, so tag and position give back the key.
 constexpr uint32_t kCellCacheBits = 11;
 constexpr uint32_t kCellCache = 1u << kCellCacheBits;
-// Per-warp buffer of claimed table slots: under 32 waiting plus one claim per lane.
-constexpr uint32_t kWarpCells = 64u;
+// Per-warp buffer of claimed table slots: under kWarpFlush waiting plus one claim
+// per lane.
+constexpr uint32_t kWarpFlush = 160u;
+constexpr uint32_t kWarpCells = kWarpFlush + 32u;
 
 // The warp's buffered slots into the batch's list of new cells, with one
 // counter atomic (a single counter bumped by every claim serialises the
@@ -1653,10 +1665,14 @@ __device__ __forceinline__ void flushWarpCells(const Dev& d, const uint32_t* wbu
 // the lane, so a run's first lane holds its lowest index; spilled points use a
 // full match), then a per-block direct-mapped cache drops a leader whose cell
 // an earlier point of the block already leads (a lower index, or any point in
-// first-come mode). Claimed slots are buffered per warp and listed 32 at a
-// time with one counter atomic.
+// first-come mode). Claimed slots are buffered per warp, and what the warps hold
+// at the end is listed with one counter atomic per block: at 32 slots a time
+// every warp met the counter, and those round trips were a third of the kernel
+// (42 us without launch overhead per 1M-point batch, 30 so; table reads alone
+// 12, claims and minimum updates the rest).
 __global__ void __launch_bounds__(256) k_vox_sample(Dev d, const Point* __restrict__ pts, uint32_t n) {
     __shared__ uint32_t s_wbuf[256 / 32][kWarpCells];
+    __shared__ uint32_t s_left[256 / 32], s_base;
     __shared__ unsigned long long s_cells[kCellCache];
     const Counters* c = d.ctr;
     if (c->batchStop || c->levelMode) return;
@@ -1741,9 +1757,9 @@ __global__ void __launch_bounds__(256) k_vox_sample(Dev d, const Point* __restri
                 cur = atomicCAS(&d.hashSlots[slot].x, kHashEmpty, key);
                 claimed = cur == kHashEmpty;
                 update = claimed || cur == key;
-                if (!update) hashInsertFrom(d, key, val, (slot + 1u) & d.hashMask);
+                if (!update) hashInsertFrom(d, key, val, nextSlot(slot, d.hashMask));
             } else {
-                hashInsertFrom(d, key, val, (slot + 1u) & d.hashMask);
+                hashInsertFrom(d, key, val, nextSlot(slot, d.hashMask));
             }
             if (update) {
                 if (lowest) atomicMin(&d.hashSlots[slot].y, val);
@@ -1756,12 +1772,25 @@ __global__ void __launch_bounds__(256) k_vox_sample(Dev d, const Point* __restri
         if (claimed) wbuf[wbufN + (uint32_t)__popc(cm & ((1u << lane) - 1u))] = slot;
         __syncwarp();
         wbufN += (uint32_t)__popc(cm);
-        if (wbufN >= 32u) {
+        if (wbufN >= kWarpFlush) {
             flushWarpCells(d, wbuf, wbufN);
             wbufN = 0;
         }
     }
-    flushWarpCells(d, wbuf, wbufN);
+    // what the warps still hold goes to the list with one counter atomic per
+    // block: one per warp queued up on the counter
+    const uint32_t warp = threadIdx.x >> 5;
+    if (lane == 0u) s_left[warp] = wbufN;
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < 256u / 32u; w++) {
+        before += w < warp ? s_left[w] : 0u;
+        all += s_left[w];
+    }
+    if (threadIdx.x == 0 && all) s_base = atomicAdd(&d.ctr->numNew, all);
+    __syncthreads();
+    for (uint32_t t = lane; t < wbufN; t += 32u) listNewCell(d, s_base + before + t, wbuf[t]);
 }
 
 // Inserts (key -> val) for k_vox_lift. Returns whether the walk goes on: it
@@ -1791,7 +1820,7 @@ __device__ __forceinline__ bool liftInsert(const Dev& d, unsigned long long key,
                 return atomicCAS(&d.hashSlots[slot].y, kHashEmpty, val) == kHashEmpty;
             }
         }
-        slot = (slot + 1u) & d.hashMask;
+        slot = nextSlot(slot, d.hashMask);
     }
     atomicOr(&d.ctr->overflowFlags, (uint32_t)kOvfBacklog);
     d.ctr->hashNeedsClear = 1u;
@@ -2044,7 +2073,7 @@ __global__ void __launch_bounds__(256) k_vox_sample_levels(Dev d, const Point* _
                     if (lowest) atomicMin(&d.hashSlots[slot[j]].y, val);
                     else atomicCAS(&d.hashSlots[slot[j]].y, kHashEmpty, val);
                 } else if (state[j] == 3u) {
-                    hashInsertFrom(d, key[j], val, (slot[j] + 1u) & d.hashMask);
+                    hashInsertFrom(d, key[j], val, nextSlot(slot[j], d.hashMask));
                 }
             }
             // the claimed slots wait in the warp's buffer; 32 or more go to the
