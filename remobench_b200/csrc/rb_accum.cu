@@ -19,11 +19,6 @@
 
 namespace rb {
 
-__device__ __forceinline__ uint32_t aq(float c, float mn, float size, float scale) {
-    float d = __fsub_rn(c, mn);
-    return __float2uint_rz(__fdiv_rn(__fmul_rn(scale, d), size));
-}
-
 // remoMortonSpread / remoMortonCode (remolod_accum.cu:24-36)
 __device__ __forceinline__ unsigned long long mortonSpread(uint32_t v) {
     unsigned long long x = (unsigned long long)v & 0xFFFFFull;
@@ -82,27 +77,65 @@ __device__ __forceinline__ void atomicAdd128(unsigned long long* lo, unsigned lo
     if (vhi + carry) atomicAdd(hi, vhi + carry);
 }
 
+// The largest fold whose chunks are cut into kAccumParts items. A warp per whole
+// chunk leaves most of the 3,552 resident warps without work below about this
+// many points (100,000 points: 18.2 us in whole chunks, 8.3 in quarters); above,
+// an item's reduction, about 20 points' worth, is better spent on a whole one.
+constexpr unsigned long long kAccumFine = 3000000ull;
+
+// Starts a fold: its counters to zero (RemolodPipeline.cpp:251-256 restarts the
+// globals per launch), and how its chunks are cut, from the points that came in
+// since the last one.
+__global__ void k_accum_begin(Dev d) {
+    Counters* c = d.ctr;
+    AccumGlobals* g = d.accumGlobals;
+    g->sumLeafCounts = 0;
+    g->pointsFolded = 0;
+    g->numLeavesFolded = 0;
+    g->innerWithSums = 0;
+    const unsigned long long seen = c->numPointsProcessed + c->spilledPointsTotal;
+    c->accumParts = seen - c->accumMark < kAccumFine ? kAccumParts : 1u;
+    c->accumMark = seen;
+    c->accumItems = 0;
+    c->mortonBound = 0;
+}
+
+// Slots per item, and the item a slot falls in: parts items per chunk.
+__device__ __forceinline__ uint32_t itemStep(const Dev& d, uint32_t parts) { return (d.ppc + parts - 1u) / parts; }
+__device__ __forceinline__ uint32_t itemOf(const Dev& d, uint32_t slot, uint32_t parts, uint32_t step) {
+    return slot / d.ppc * parts + slot % d.ppc / step;
+}
+
+__device__ __forceinline__ unsigned long long mortonCode(uint32_t x, uint32_t y, uint32_t z) {
+    return (mortonSpread(x) << 2) | (mortonSpread(y) << 1) | mortonSpread(z);
+}
+
 // The fold's plan: the nodes to visit (the dirty list, or every node), each
 // leaf's new range [count, min(numPoints, capacity)) read before any fold
 // updates count, and each node's work items. An inner node with sums is one
-// item (cleared); a leaf with new points one item per point chunk its new
-// range touches. Sums are exact, so the order of items is free: each block
+// item (cleared); a leaf with new points one item per point chunk, or part of
+// one (Counters::accumParts), its new range touches. Sums are exact, so the order of items is free: each block
 // claims a contiguous run of item indices with one atomic (Counters::
-// accumItems, zeroed before the launch) and writes every item's plan entry,
+// accumItems) and writes every item's plan entry,
 // so a warp of the fold finds its item with one load. Items can pass
 // accumUnitCap (every live point chunk plus every node) only once the arena
 // has run out (RB_OVF_ARENA): those are not folded. Folded-leaf and point
-// totals are added per block.
+// totals are added per block. The watermark needs only the leaves that can hold
+// the largest Morton code: a code grows with each coordinate, so a point's is at
+// least its leaf's lower corner's (clamping only raises a coordinate), and the
+// largest lower corner of the leaves with new points bounds it from below.
 __global__ void __launch_bounds__(256) k_accum_plan(Dev d, int useList) {
     __shared__ uint32_t s_warp[8];
     __shared__ uint32_t s_base, s_leaves;
-    __shared__ unsigned long long s_points;
+    __shared__ unsigned long long s_points, s_bound;
     Counters* c = d.ctr;
+    const uint32_t parts = c->accumParts, step = itemStep(d, parts);
     const uint32_t total = useList ? (c->numDirty < d.maxNodes ? c->numDirty : d.maxNodes) : c->numNodes;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
         s_leaves = 0;
         s_points = 0;
+        s_bound = 0;
     }
     __syncthreads();
     // the same number of steps in every thread of the block
@@ -119,7 +152,9 @@ __global__ void __launch_bounds__(256) k_accum_plan(Dev d, int useList) {
                 const uint32_t np = d.numPoints[node];
                 to = np < cap ? np : cap;
                 if (to > from) {
-                    items = (to - 1u) / d.ppc - from / d.ppc + 1u;
+                    items = itemOf(d, to - 1u, parts, step) - itemOf(d, from, parts, step) + 1u;
+                    const uint32_t sh = (uint32_t)kMaxDepth - d.level[node];
+                    atomicMax(&s_bound, mortonCode(d.nodeX[node] << sh, d.nodeY[node] << sh, d.nodeZ[node] << sh));
                     atomicAdd(&s_leaves, 1u);
                     atomicAdd(&s_points, (unsigned long long)(to - from));
                 } else {
@@ -160,6 +195,8 @@ __global__ void __launch_bounds__(256) k_accum_plan(Dev d, int useList) {
         atomicAdd(&d.accumGlobals->numAccumulated, s_points);
         atomicAdd(&d.accumGlobals->pointsFolded, (uint32_t)s_points);
         atomicAdd(&d.accumGlobals->numLeavesFolded, s_leaves);
+        // past an arena overflow a chunk may be missing, and its points with it
+        if (!(c->overflowFlags & (uint32_t)kOvfArena)) atomicMax(&c->mortonBound, s_bound);
     }
 }
 
@@ -178,13 +215,16 @@ __device__ __forceinline__ void add128pair(unsigned long long& lo, unsigned long
 // warp issues the atomic of sum k, so an item's 21 updates go out together.
 // The watermark is merged per block in shared memory, one global atomic per
 // block. Three blocks per SM (80 registers, a few bytes spilled) fold 9% faster
-// than the two that 93 registers allow.
+// than the two that 93 registers allow. Bound by instruction issue: 20M points
+// took 108 us with a division per coordinate, 64-bit clamps and a Morton
+// comparison per point, 77 us without (4.2 TB/s of the points read).
 __global__ void __launch_bounds__(kAccumThreads, 3) k_accumulate(Dev d, uint32_t batchIndex, int useList) {
     __shared__ unsigned long long s_morton;
     const Counters* c = d.ctr;
     const uint32_t items = c->accumItems;
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t ppc = d.ppc;
+    const uint32_t ppc = d.ppc, parts = c->accumParts, step = itemStep(d, parts);
+    const unsigned long long bound = c->mortonBound;
     if (threadIdx.x == 0) s_morton = 0ull;
     __syncthreads();
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
@@ -202,16 +242,19 @@ __global__ void __launch_bounds__(kAccumThreads, 3) k_accumulate(Dev d, uint32_t
             }
             continue;
         }
-        const uint32_t ci = from0 / ppc + (it - d.accumItem[w]);
-        const uint32_t from = from0 > ci * ppc ? from0 : ci * ppc;
-        const uint32_t end = to < (ci + 1u) * ppc ? to : (ci + 1u) * ppc;
+        const uint32_t part = itemOf(d, from0, parts, step) + (it - d.accumItem[w]);
+        const uint32_t ci = part / parts, lo = ci * ppc + part % parts * step;
+        const uint32_t from = max(from0, lo);
+        const uint32_t end = min(to, min(lo + step, (ci + 1u) * ppc));
         const uint32_t lv = d.level[node];
         const uint32_t sh = 28u - lv;
-        const long long lim = 1ll << sh;
-        const long long bx = (long long)d.nodeX[node] << sh;
-        const long long by = (long long)d.nodeY[node] << sh;
-        const long long bz = (long long)d.nodeZ[node] << sh;
+        const uint32_t lim = 1u << sh;
+        const uint32_t origin[3] = {d.nodeX[node] << sh, d.nodeY[node] << sh, d.nodeZ[node] << sh};
         const uint32_t phys = d.tablePool[d.ptTableOff[node] + ci];
+        // whether a point of this leaf can hold the watermark (k_accum_plan)
+        const uint32_t sh20 = (uint32_t)kMaxDepth - lv, corner = (1u << sh20) - 1u;
+        const bool candidate = mortonCode((d.nodeX[node] << sh20) | corner, (d.nodeY[node] << sh20) | corner,
+                                          (d.nodeZ[node] << sh20) | corner) >= bound;
 
         // Per lane at most ppc / 32 + 1 points: Σq < 2^28 · 32 needs u64, Σq·q <
         // 32 · 2^56 fits u64 without carries, colour sums fit u32; the 128-bit
@@ -237,15 +280,12 @@ __global__ void __launch_bounds__(kAccumThreads, 3) k_accumulate(Dev d, uint32_t
                 for (int h = 0; h < 4; h++) {
                     if (!ok[h]) continue;
                     const float4 v = v4[h];
-                    const uint32_t P[3] = {aq(v.x, d.boxMin[0], d.octreeSize, 268435456.0f),
-                                           aq(v.y, d.boxMin[1], d.octreeSize, 268435456.0f),
-                                           aq(v.z, d.boxMin[2], d.octreeSize, 268435456.0f)};
+                    const uint32_t P[3] = {quant28(d, v.x, 0), quant28(d, v.y, 1), quant28(d, v.z, 2)};
                     // clamped to [0, 2^(28 - level)]: 32-bit values, 64-bit products
                     uint32_t q[3];
-                    const long long r[3] = {(long long)P[0] - bx, (long long)P[1] - by, (long long)P[2] - bz};
 #pragma unroll
                     for (int k = 0; k < 3; k++) {
-                        q[k] = (uint32_t)(r[k] < 0 ? 0 : (r[k] > lim ? lim : r[k]));
+                        q[k] = min(max(P[k], origin[k]) - origin[k], lim);
                         s1[k] += q[k];
                     }
                     p2[0] += (unsigned long long)q[0] * q[0];
@@ -261,24 +301,28 @@ __global__ void __launch_bounds__(kAccumThreads, 3) k_accumulate(Dev d, uint32_t
                         c1[k] += ch[k];
                         c2[k] += ch[k] * ch[k];
                     }
-                    // the 20-bit coordinate is the 28-bit one shifted (power-of-two scaling
-                    // commutes with round-to-nearest); only a saturated conversion differs
-                    uint32_t X = P[0] < 0xFFFFFF00u ? P[0] >> 8 : aq(v.x, d.boxMin[0], d.octreeSize, 1048576.0f);
-                    uint32_t Y = P[1] < 0xFFFFFF00u ? P[1] >> 8 : aq(v.y, d.boxMin[1], d.octreeSize, 1048576.0f);
-                    uint32_t Z = P[2] < 0xFFFFFF00u ? P[2] >> 8 : aq(v.z, d.boxMin[2], d.octreeSize, 1048576.0f);
-                    X = X < 1048575u ? X : 1048575u;
-                    Y = Y < 1048575u ? Y : 1048575u;
-                    Z = Z < 1048575u ? Z : 1048575u;
-                    if (mortonLess(mx, my, mz, X, Y, Z)) {
-                        mx = X;
-                        my = Y;
-                        mz = Z;
+                    // only where it can be the largest: in the last leaves in Morton
+                    // order, or past the box, where a leaf's cube says nothing of it
+                    if (candidate || max(max(P[0], P[1]), P[2]) >= (1u << 28)) {
+                        // the 20-bit coordinate is the 28-bit one shifted (power-of-two scaling
+                        // commutes with round-to-nearest); only a saturated conversion differs
+                        uint32_t X = P[0] < 0xFFFFFF00u ? P[0] >> 8 : quant20(d, v.x, 0);
+                        uint32_t Y = P[1] < 0xFFFFFF00u ? P[1] >> 8 : quant20(d, v.y, 1);
+                        uint32_t Z = P[2] < 0xFFFFFF00u ? P[2] >> 8 : quant20(d, v.z, 2);
+                        X = X < 1048575u ? X : 1048575u;
+                        Y = Y < 1048575u ? Y : 1048575u;
+                        Z = Z < 1048575u ? Z : 1048575u;
+                        if (mortonLess(mx, my, mz, X, Y, Z)) {
+                            mx = X;
+                            my = Y;
+                            mz = Z;
+                        }
                     }
                 }
             }
         }
         // the warp's sums: 21 values (s1 x3, s2 lo/hi x6, c1 x3, c2 x3) and the watermark
-        unsigned long long wm = (mortonSpread(mx) << 2) | (mortonSpread(my) << 1) | mortonSpread(mz);
+        unsigned long long wm = mortonCode(mx, my, mz);
         unsigned long long lo2[6], hi2[6] = {0, 0, 0, 0, 0, 0};
         unsigned long long c1w[3], c2w[3];
 #pragma unroll
@@ -342,9 +386,14 @@ __global__ void __launch_bounds__(kAccumThreads, 3) k_accumulate(Dev d, uint32_t
     if (threadIdx.x == 0 && s_morton != 0ull) atomicMax(&d.accumGlobals->mortonWatermark, s_morton);
 }
 
-// kernel_accum_verify (remolod_accum.cu:214-233)
+// kernel_accum_verify (remolod_accum.cu:214-233). One thread restarts the dirty
+// list, which names the nodes touched since this fold (nothing here reads it).
 __global__ void __launch_bounds__(256) k_accum_verify(Dev d) {
     const uint32_t nn = d.ctr->numNodes;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        d.ctr->buildStamp += 1u;
+        d.ctr->numDirty = 0;
+    }
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
         const uint32_t cnt = d.accum[i].count;
         if (leafRow(d, i)) {
@@ -356,8 +405,8 @@ __global__ void __launch_bounds__(256) k_accum_verify(Dev d) {
 }
 
 void launchAccumulate(const Dev& d, uint32_t batchIndex, int useList, int grid, cudaStream_t s) {
-    cudaMemsetAsync(&d.ctr->accumItems, 0, sizeof(uint32_t), s);
-    k_accum_plan<<<grid, 256, 0, s>>>(d, useList);
+    k_accum_begin<<<1, 1, 0, s>>>(d);
+    k_accum_plan<<<grid / 4 + 1, 256, 0, s>>>(d, useList);
     k_accumulate<<<grid, kAccumThreads, 0, s>>>(d, batchIndex, useList);
 }
 void launchAccumVerify(const Dev& d, int grid, cudaStream_t s) { k_accum_verify<<<grid, 256, 0, s>>>(d); }

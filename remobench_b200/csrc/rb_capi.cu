@@ -324,12 +324,8 @@ rb_status uploadRing(rb_ctx* c) {
 
 rb_status accumulate(rb_ctx* c, uint32_t batchIndex) {
     const Dev& d = c->d;
-    // sumLeafCounts .. innerWithSums restart per launch (RemolodPipeline.cpp:251-256)
-    RB_CUDA(c, cudaMemsetAsync(reinterpret_cast<uint8_t*>(d.accumGlobals) + 16, 0, 20, c->stream));
     LAUNCH(c, K_ACCUMULATE, 0, rb::launchAccumulate(d, batchIndex, c->accumAll ? 0 : 1, c->numSMs * 8, c->stream));
     LAUNCH(c, K_ACCUM_VERIFY, 0, rb::launchAccumVerify(d, c->numSMs * 2, c->stream));
-    // the dirty list restarts: it names the nodes touched since this fold
-    LAUNCH(c, K_BUILD_BEGIN, 1, (k_build_begin<<<1, 1, 0, c->stream>>>(c->d.ctr)));
     RB_CUDA(c, cudaGetLastError());
     c->accumAll = false;
     return RB_OK;
@@ -494,6 +490,8 @@ rb_status rb_allocate(rb_ctx* c, const rb_cloud_meta* meta, uint64_t budget) {
                 sz = meta->box_max[2] - meta->box_min[2];
     d.octreeSize = std::max(std::max(sx, sy), sz);
     if (!(d.octreeSize > 0.0f)) return fail(c, RB_ERR_INVALID_ARG, "empty bounding box");
+    // sizes whose quotients' residuals stay normal (rb_state.h, quotient)
+    d.octreeRecip = d.octreeSize >= 0x1p-40f && d.octreeSize <= 0x1p40f ? 1.0f / d.octreeSize : 0.0f;
 
     if (cfg.pipeline == RB_PIPELINE_FLAT) {
         // flat keeps no tree: render scratch only
@@ -598,7 +596,7 @@ rb_status rb_allocate(rb_ctx* c, const rb_cloud_meta* meta, uint64_t budget) {
     ALLOC(d.accumFrom, N, "accumulate plan ranges");
     ALLOC(d.accumTo, N, "accumulate plan ranges");
     ALLOC(d.accumItem, (uint64_t)N + 1, "accumulate plan items");
-    d.accumUnitCap = (uint32_t)std::min<uint64_t>((uint64_t)d.maxPtChunks + N, UINT32_MAX);
+    d.accumUnitCap = (uint32_t)std::min<uint64_t>((uint64_t)d.maxPtChunks * rb::kAccumParts + N, UINT32_MAX);
     ALLOC(d.accumUnitW, d.accumUnitCap, "accumulate work items");
     ALLOC(d.hist8, (uint64_t)N * 8, "child-octant counts");
     ALLOC(d.arrive, N, "points reaching each leaf");

@@ -33,11 +33,6 @@ namespace rb {
 
 namespace {
 
-__device__ __forceinline__ uint32_t quant28r(float c, float mn, float size) {
-    const float d = __fsub_rn(c, mn);
-    return __float2uint_rz(__fdiv_rn(__fmul_rn(268435456.0f, d), size));
-}
-
 __device__ __forceinline__ uint32_t cellOf(uint32_t x28, uint32_t y28, uint32_t z28, uint32_t level) {
     const uint32_t sh = (uint32_t)kMaxDepth + 1u - level;
     return ((x28 >> sh) & 127u) + ((y28 >> sh) & 127u) * 128u + ((z28 >> sh) & 127u) * 16384u;
@@ -305,9 +300,9 @@ __global__ void __launch_bounds__(256) k_cf_gather(Dev d, RefineScratch r) {
             for (uint32_t j = 0; j < 4u; j++) {
                 const float4 p = j == 0u ? v[0] : (j == 1u ? v[1] : (j == 2u ? v[2] : v[3]));
                 const bool there = j == 0u ? ok[0] : (j == 1u ? ok[1] : (j == 2u ? ok[2] : ok[3]));
-                const uint32_t x = quant28r(p.x, d.boxMin[0], d.octreeSize),
-                               y = quant28r(p.y, d.boxMin[1], d.octreeSize),
-                               z = quant28r(p.z, d.boxMin[2], d.octreeSize);
+                const uint32_t x = quant28(d, p.x, 0),
+                               y = quant28(d, p.y, 1),
+                               z = quant28(d, p.z, 2);
                 const uint32_t color = __float_as_uint(p.w);
                 uint32_t cr = color & 255u, cg = (color >> 8) & 255u, cb = (color >> 16) & 255u, n = 1u;
                 const bool regular = max(max(x, y), z) <= (1u << 28);

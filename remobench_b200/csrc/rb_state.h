@@ -90,6 +90,9 @@ struct Counters {
     uint32_t hashNeedsClear;      // the cell table holds entries its list cannot name
     uint32_t callBatches;         // batches built since the build call began
     uint32_t accumItems;          // work items of the current Accumulate launch
+    uint32_t accumParts;          // items a point chunk is cut into (k_accum_begin)
+    unsigned long long accumMark;   // points processed and spilled when the last Accumulate began
+    unsigned long long mortonBound; // no new point's leaf with a Morton code above this is left out of the watermark
     uint32_t numZero;             // grids of nodes split this batch, to zero after expand
     uint32_t histValid;           // hist8 holds the child-octant counts of the nodes to split next
     uint32_t countLo, countHi;    // nodes [countLo, countHi) whose points the next recount counts
@@ -244,7 +247,7 @@ struct Dev {
     uint32_t* accumTo;       // [maxNodes]
     uint32_t* accumItem;     // [maxNodes + 1] exclusive prefix of work items
     uint32_t* accumUnitW;    // [accumUnitCap] plan entry of each work item
-    uint32_t accumUnitCap;   // point chunks + nodes: every fold's items fit
+    uint32_t accumUnitCap;   // kAccumParts per point chunk + nodes: every fold's items fit
     uint32_t* zeroList;      // [zeroCap] grids to zero after the expand loop
     // per node, its points per child octant, counted by the recount for the
     // nodes made by the last split: one level of lookahead for the next split
@@ -285,7 +288,10 @@ struct Dev {
     uint64_t safetyMargin;
     float boxMin[3];
     float octreeSize;
+    float octreeRecip;       // 1 / octreeSize rounded to nearest, 0: divide (see quotient)
 };
+
+constexpr uint32_t kAccumParts = 4;  // items a chunk is cut into when a fold is small
 
 constexpr uint32_t kGridUnits = (uint32_t)(kGridBytes / 16u);
 
@@ -310,6 +316,35 @@ __device__ __forceinline__ uint32_t* chunkIndices(const Dev& d, uint32_t phys) {
 __device__ __forceinline__ uint32_t* gridWordsAt(const Dev& d, uint32_t g) {
     return reinterpret_cast<uint32_t*>(d.arena + (uint64_t)g * 16u);
 }
+// a / octreeSize, rounded to nearest as the division rounds it, for the points'
+// coordinates: two residual corrections of a * (1 / octreeSize) with fused
+// multiply-adds (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34(1), 1990: a quotient within one
+// unit in the last place, corrected by its exact residual times the correctly
+// rounded reciprocal, is the rounded quotient; the first correction brings it
+// within one unit). The host allows it (octreeRecip != 0) for sizes whose
+// reciprocal and residuals stay normal; quotients that do not fit an unsigned
+// integer are not corrected (they saturate), and those below one may round
+// differently far below their truncation to zero. Five instructions and no
+// branch instead of the division's call-out: three of them per point in every
+// kernel that quantises. Compared with the division for every float at six sizes
+// and every mantissa at 74: the same integers. Where issue bounds it shows
+// (k_accumulate, 20M points: 108 -> 95 us); the kernels of a batch wait on memory.
+__device__ __forceinline__ float quotient(const Dev& d, float a) {
+    const float y = d.octreeRecip;
+    if (y == 0.0f) return __fdiv_rn(a, d.octreeSize);
+    const float q0 = __fmul_rn(a, y);
+    const float q1 = __fmaf_rn(__fmaf_rn(-d.octreeSize, q0, a), y, q0);
+    const float q2 = __fmaf_rn(__fmaf_rn(-d.octreeSize, q1, a), y, q1);
+    return fabsf(q0) < 8.0e9f ? q2 : q0;
+}
+// The octree coordinate of `c` on a 2^20 or 2^28 grid (scale), saturating.
+__device__ __forceinline__ uint32_t quantise(const Dev& d, float c, int axis, float scale) {
+    return __float2uint_rz(quotient(d, __fmul_rn(scale, __fsub_rn(c, d.boxMin[axis]))));
+}
+__device__ __forceinline__ uint32_t quant20(const Dev& d, float c, int axis) { return quantise(d, c, axis, 1048576.0f); }
+__device__ __forceinline__ uint32_t quant28(const Dev& d, float c, int axis) { return quantise(d, c, axis, 268435456.0f); }
+
 // A slot's chunk and its place in it: slot / ppc and slot % ppc through the
 // rounded-down reciprocal (Dev::ppcRecip), whose quotient is at most one low.
 __device__ __forceinline__ uint32_t chunkOf(const Dev& d, uint32_t slot, uint32_t& within) {

@@ -19,16 +19,6 @@
 
 namespace rb {
 
-__device__ __forceinline__ uint32_t quant20(float c, float mn, float size) {
-    float d = __fsub_rn(c, mn);
-    return __float2uint_rz(__fdiv_rn(__fmul_rn(1048576.0f, d), size));
-}
-
-__device__ __forceinline__ uint32_t quant28(float c, float mn, float size) {
-    float d = __fsub_rn(c, mn);
-    return __float2uint_rz(__fdiv_rn(__fmul_rn(268435456.0f, d), size));
-}
-
 __device__ __forceinline__ Point loadPoint(const Point* p) {
     float4 v = __ldg(reinterpret_cast<const float4*>(p));
     Point q;
@@ -281,9 +271,9 @@ __global__ void __launch_bounds__(256) k_count_first(Dev d, const Point* __restr
         uint32_t leaf = kNone;
         if (i < end) {
             const Point p = loadPoint(pts + i);
-            leaf = descendFromRoot(d, quant20(p.x, d.boxMin[0], d.octreeSize),
-                                   quant20(p.y, d.boxMin[1], d.octreeSize),
-                                   quant20(p.z, d.boxMin[2], d.octreeSize));
+            leaf = descendFromRoot(d, quant20(d, p.x, 0),
+                                   quant20(d, p.y, 1),
+                                   quant20(d, p.z, 2));
             d.leafOf[i] = leaf;
         }
         blockCountAt<false>(d, s_counts, leaf);
@@ -336,9 +326,9 @@ __device__ __forceinline__ void recountBody(const Dev& d, const Point* __restric
             uint32_t cur = batchPt ? d.leafOf[i] : d.spillLeaf[i - n];
             if (d.splitIter[cur] == prevStamp) {
                 const Point p = batchPt ? loadPoint(pts + i) : d.spillPts[i - n];
-                const uint32_t x = quant20(p.x, d.boxMin[0], d.octreeSize),
-                               y = quant20(p.y, d.boxMin[1], d.octreeSize),
-                               z = quant20(p.z, d.boxMin[2], d.octreeSize);
+                const uint32_t x = quant20(d, p.x, 0),
+                               y = quant20(d, p.y, 1),
+                               z = quant20(d, p.z, 2);
                 uint32_t lv = d.level[cur];
                 while (lv < (uint32_t)kMaxDepth) {
                     const int32_t nx = d.child[cur * 8u + childIndex(x, y, z, lv)];
@@ -1181,9 +1171,9 @@ __device__ __forceinline__ void deepBin(const Dev& d, DeepBlockBins& bins, bool 
                                         const Point& p, uint32_t levels, uint32_t* codeOut) {
     uint32_t x = 0, y = 0, z = 0;
     if (active) {
-        x = quant20(p.x, d.boxMin[0], d.octreeSize);
-        y = quant20(p.y, d.boxMin[1], d.octreeSize);
-        z = quant20(p.z, d.boxMin[2], d.octreeSize);
+        x = quant20(d, p.x, 0);
+        y = quant20(d, p.y, 1);
+        z = quant20(d, p.z, 2);
     }
     uint32_t code = 0;
 #pragma unroll
@@ -1466,9 +1456,9 @@ __device__ void finishLeavesBody(const Dev& d, const Point* __restrict__ pts, ui
             leaf = batchPt ? d.leafOf[i] : d.spillLeaf[i - n];
             if (stale) {
                 const Point p = batchPt ? loadPoint(pts + i) : d.spillPts[i - n];
-                const uint32_t x = quant20(p.x, d.boxMin[0], d.octreeSize),
-                               y = quant20(p.y, d.boxMin[1], d.octreeSize),
-                               z = quant20(p.z, d.boxMin[2], d.octreeSize);
+                const uint32_t x = quant20(d, p.x, 0),
+                               y = quant20(d, p.y, 1),
+                               z = quant20(d, p.z, 2);
                 const uint32_t from = leaf;
                 uint32_t lv = d.level[leaf];
                 while (lv < (uint32_t)kMaxDepth) {
@@ -1717,9 +1707,9 @@ __global__ void __launch_bounds__(256) k_vox_sample(Dev d, const Point* __restri
                 tl = lv - 1u;
             }
             if (g != kNone) {
-                const uint32_t x28 = quant28(p.x, d.boxMin[0], d.octreeSize);
-                const uint32_t y28 = quant28(p.y, d.boxMin[1], d.octreeSize);
-                const uint32_t z28 = quant28(p.z, d.boxMin[2], d.octreeSize);
+                const uint32_t x28 = quant28(d, p.x, 0);
+                const uint32_t y28 = quant28(d, p.y, 1);
+                const uint32_t z28 = quant28(d, p.z, 2);
                 const uint32_t vi = cellAt(x28, y28, z28, tl);
                 if (((__ldg(gridWordsAt(d, g) + (vi >> 5)) >> (vi & 31u)) & 1u) == 0u)
                     key = ((unsigned long long)node << 21) | (unsigned long long)vi;
@@ -1962,9 +1952,9 @@ __global__ void __launch_bounds__(256) k_vox_sample_levels(Dev d, const Point* _
         }
         uint32_t x28 = 0, y28 = 0, z28 = 0, lv = 0;
         if (active) {
-            x28 = quant28(p.x, d.boxMin[0], d.octreeSize);
-            y28 = quant28(p.y, d.boxMin[1], d.octreeSize);
-            z28 = quant28(p.z, d.boxMin[2], d.octreeSize);
+            x28 = quant28(d, p.x, 0);
+            y28 = quant28(d, p.y, 1);
+            z28 = quant28(d, p.z, 2);
             lv = d.level[leaf];
         }
         // (1) which levels' cells were empty before this batch
@@ -2416,9 +2406,10 @@ __global__ void __launch_bounds__(256) k_vox_store(Dev d) {
         const float mny = __fmaf_rn((float)d.nodeY[node], nodeSize, d.boxMin[1]);
         const float mnz = __fmaf_rn((float)d.nodeZ[node], nodeSize, d.boxMin[2]);
         Point v;
-        v.x = __fadd_rn(mnx, __fdiv_rn(__fmul_rn(nodeSize, __fadd_rn((float)px, 0.5f)), 128.0f));
-        v.y = __fadd_rn(mny, __fdiv_rn(__fmul_rn(nodeSize, __fadd_rn((float)py, 0.5f)), 128.0f));
-        v.z = __fadd_rn(mnz, __fdiv_rn(__fmul_rn(nodeSize, __fadd_rn((float)pz, 0.5f)), 128.0f));
+        // 0.0078125 = 1 / 128: the same rounding as the division
+        v.x = __fadd_rn(mnx, __fmul_rn(__fmul_rn(nodeSize, __fadd_rn((float)px, 0.5f)), 0.0078125f));
+        v.y = __fadd_rn(mny, __fmul_rn(__fmul_rn(nodeSize, __fadd_rn((float)py, 0.5f)), 0.0078125f));
+        v.z = __fadd_rn(mnz, __fmul_rn(__fmul_rn(nodeSize, __fadd_rn((float)pz, 0.5f)), 0.0078125f));
         v.color = d.hashNewColor[e];
         if (s < d.numVoxelChunks[node] * ppc) {
             const uint32_t phys = d.tablePool[d.vxTableOff[node] + s / ppc];
