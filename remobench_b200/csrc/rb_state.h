@@ -258,8 +258,8 @@ struct Dev {
     uint32_t* arrive;        // [maxNodes]
     // multi-level expand round: per root slot, the points below it counted at
     // every depth 1..kDeepLevels ([kDeepRoots][kDeepCells]); per root node its
-    // slot; per node made by the round, (slot << 16) | its code below the root;
-    // per generation, the nodes split in id order
+    // slot; per node made by the round, its depth, slot and code below the root
+    // (deepMetaOf); per generation, the nodes split in id order, from deepBase
     uint32_t* deepCnt;
     uint32_t* deepNode;      // [kDeepRoots * kDeepCells] the node the round made for each cube, kNone elsewhere
     uint32_t* moveCode;      // [slot capacity] each binned batch point's cube code at the round's deepest depth

@@ -916,50 +916,6 @@ __global__ void __launch_bounds__(256) k_spill_copy(Dev d, uint32_t gated) { spi
 // spilling node) go on through the per-iteration passes, as do batches whose
 // first count lists more than kDeepRoots nodes or a node at the deepest level.
 
-// A new node: child `i` of `parent` at id `ch` (doSplitting's child set-up,
-// remolod_octree.cu:323-347), with its ancestor row.
-__device__ __forceinline__ void makeChild(const Dev& d, uint32_t ch, uint32_t parent, uint32_t i) {
-    // the parent's fields and its whole ancestor row in one round of loads
-    // (row entries at and past its level are read and ignored)
-    const uint32_t plv = d.level[parent], pg = d.grid[parent];
-    const uint32_t px = d.nodeX[parent], py = d.nodeY[parent], pz = d.nodeZ[parent];
-    const uint2* prow = d.anc + (size_t)parent * kMaxDepth;
-    uint2 arow[kMaxDepth];
-#pragma unroll
-    for (uint32_t l = 0; l < (uint32_t)kMaxDepth; l++) arow[l] = prow[l];
-    const uint32_t lv = plv + 1u;
-#pragma unroll
-    for (int q = 0; q < 8; q++) d.child[ch * 8u + q] = -1;
-    d.counter[ch] = 0;
-    reinterpret_cast<uint4*>(d.hist8 + (size_t)ch * 8u)[0] = make_uint4(0, 0, 0, 0);
-    reinterpret_cast<uint4*>(d.hist8 + (size_t)ch * 8u)[1] = make_uint4(0, 0, 0, 0);
-    d.numPoints[ch] = 0;
-    d.level[ch] = lv;
-    d.nodeX[ch] = 2u * px + ((i >> 2) & 1u);
-    d.nodeY[ch] = 2u * py + ((i >> 1) & 1u);
-    d.nodeZ[ch] = 2u * pz + (i & 1u);
-    d.grid[ch] = kNone;
-    d.numVoxels[ch] = 0;
-    d.numVoxelsStored[ch] = 0;
-    d.numPointChunks[ch] = 0;
-    d.numVoxelChunks[ch] = 0;
-    d.ptTableOff[ch] = kNone;
-    d.ptTableCap[ch] = 0;
-    d.vxTableOff[ch] = kNone;
-    d.vxTableCap[ch] = 0;
-    d.splitIter[ch] = 0;
-    d.dirtyStamp[ch] = 0;
-    AccumI z = {};
-    d.accum[ch] = z;
-    uint2* crow = d.anc + (size_t)ch * kMaxDepth;
-#pragma unroll
-    for (uint32_t l = 0; l < (uint32_t)kMaxDepth; l++)
-        if (l + 1u < lv) crow[l] = arow[l];
-    crow[lv - 1u] = make_uint2(parent, pg);
-    d.parent[ch] = make_uint2(parent, pg);
-    d.child[parent * 8u + i] = (int32_t)ch;
-}
-
 // The bookkeeping every split shares: a grid if the node has none (allocated
 // once, zeroed at every split, :365-387), its split stamp, the grid on the
 // zero list and the node on the dirty list.
@@ -1271,6 +1227,16 @@ __global__ void __launch_bounds__(256) k_deep_bin(Dev d, const Point* __restrict
     deepBinsFlush(d, s_bins);
 }
 
+// A node made by the round: its depth below its root (from bit 28), its root's
+// slot (from bit 16) and its cube code (three bits a depth).
+__device__ __forceinline__ uint32_t deepMetaOf(uint32_t depth, uint32_t slot, uint32_t code) {
+    return (depth << 28) | (slot << 16) | code;
+}
+__device__ __forceinline__ uint32_t metaDepth(uint32_t m) { return m >> 28; }
+__device__ __forceinline__ uint32_t metaSlot(uint32_t m) { return (m >> 16) & 0xFFFu; }
+__device__ __forceinline__ uint32_t metaCode(uint32_t m) { return m & 0xFFFFu; }
+static_assert(kDeepRoots <= 4096u && 3u * kDeepLevels <= 16u, "deepMeta's fields");
+
 // Iterations 2 .. 1 + kDeepLevels from the binned counts: generation g (the
 // nodes made by iteration g's splits, g >= 1) is counted in iteration g + 1;
 // its nodes over the limit split in that iteration, in increasing id, each
@@ -1279,39 +1245,61 @@ __global__ void __launch_bounds__(256) k_deep_bin(Dev d, const Point* __restrict
 // nothing or at the pass limit. Nodes of the last generation counted and
 // still over the limit are handed to the per-iteration passes. One block of
 // 1024 threads.
+//
+// Bound by its chain of dependent round trips, a few per generation, so each
+// generation does only what the next needs: the counts, the ids, and the split
+// nodes' grids and list places. The counters those come from belong to this
+// block while it runs, so they are read once, advanced by the scan's prefixes
+// and written once; a new node has no grid and is on no list, so nothing of it
+// is read. The rest of a node follows from its record alone and is written by
+// k_deep_move's warps (initDeepNode). 17 us per batch with every child set up
+// from its parent's row and an atomic per list and split, 8.7 us so, with 1.3 us
+// more in k_deep_move.
+constexpr uint32_t kDeepCached = 4096;  // records and split nodes kept in shared memory
+
 __global__ void __launch_bounds__(1024) k_deep_split(Dev d) {
     __shared__ uint32_t s_warp[32];
+    __shared__ uint32_t s_meta[kDeepCached];
+    __shared__ uint32_t s_par[kDeepCached / 8u];
     Counters* c = d.ctr;
     if (c->batchStop || !c->deepActive) return;
     const uint32_t roots = c->deepRoots, levels = c->deepLevels, base = c->deepBase, it0 = c->iter;
-    const uint32_t batchTag = c->batchletIndex << 5;
+    const uint32_t batchTag = c->batchletIndex << 5, buildStamp = c->buildStamp;
+    const uint32_t pool = c->gridPoolSize, taken0 = c->gridPoolTaken, bump0 = c->arenaBump;
+    const uint32_t zero0 = c->numZero, dirty0 = c->numDirty;
+    // the parents' records and the split list, past what shared memory holds in
+    // global memory
+    auto metaAt = [&](uint32_t k) { return k < kDeepCached ? s_meta[k] : d.deepMeta[k]; };
+    auto make = [&](uint32_t k, uint32_t meta) {
+        d.deepMeta[k] = meta;
+        if (k < kDeepCached) s_meta[k] = meta;
+        d.deepNode[(size_t)metaSlot(meta) * kDeepCells + deepOffset(metaDepth(meta)) + metaCode(meta)] = base + k;
+        d.counter[base + k] = 0;
+    };
     // generation 1: the roots' children, 8 consecutive ids per root in slot order
-    for (uint32_t t = threadIdx.x; t < 8u * roots; t += blockDim.x) {
-        makeChild(d, base + t, d.splitRecs[t >> 3].node, t & 7u);
-        d.deepMeta[t] = ((t >> 3) << 16) | (t & 7u);
-        d.deepNode[(size_t)(t >> 3) * kDeepCells + deepOffset(1u) + (t & 7u)] = base + t;
-    }
+    for (uint32_t t = threadIdx.x; t < 8u * roots; t += blockDim.x) make(t, deepMetaOf(1u, t >> 3, t & 7u));
     __syncthreads();
-    uint32_t lo = base, hi = base + 8u * roots;
-    uint32_t splits = 0, itEnd = 0, cont = 0;
+    uint32_t lo = 0, hi = 8u * roots;  // the generation, from base
+    uint32_t splits = 0, arenaGrids = 0, itEnd = 0, cont = 0;
+    bool arenaFull = false;
     for (uint32_t g = 1;; g++) {
         const uint32_t it = it0 + g;  // the iteration that counts generation g
         if (it > d.maxExpandIters) {
             itEnd = it;  // the loop ended after the split that made generation g
             break;
         }
-        const uint32_t room = d.maxNodes > hi ? (d.maxNodes - hi) / 8u : 0u;
+        const uint32_t room = d.maxNodes > base + hi ? (d.maxNodes - base - hi) / 8u : 0u;
         // running totals, the same in every thread (the scan returns them to all)
         uint32_t want = 0, contRun = 0;
         for (uint32_t t0 = lo; t0 < hi; t0 += blockDim.x) {
-            const uint32_t node = t0 + threadIdx.x;
+            const uint32_t k = t0 + threadIdx.x;
             uint32_t cnt = 0;
-            if (node < hi) {
-                const uint32_t meta = d.deepMeta[node - base];
-                cnt = deepCount(d, meta >> 16, g, meta & 0xFFFFu, levels);
-                d.counter[node] = cnt;
+            if (k < hi) {
+                const uint32_t meta = metaAt(k);
+                cnt = deepCount(d, metaSlot(meta), g, metaCode(meta), levels);
+                d.counter[base + k] = cnt;
             }
-            const bool over = node < hi && cnt > d.maxPointsPerNode;
+            const bool over = k < hi && cnt > d.maxPointsPerNode;
             const uint32_t wantSplit = (over && g < levels) ? 1u : 0u;
             const uint32_t wantCont = (over && g == levels) ? 1u : 0u;
             // one scan for both lists: splits in the low half, continuations
@@ -1320,11 +1308,29 @@ __global__ void __launch_bounds__(1024) k_deep_split(Dev d) {
             const uint32_t pre = blockExclusiveScan(wantSplit | (wantCont << 16), &tot, s_warp);
             const uint32_t j = want + (pre & 0xFFFFu);
             if (wantSplit && j < room) {
-                bookSplit(d, c, node, batchTag | it);
-                d.deepPar[j] = node;
+                // its grid: a collapsed node's from the pool while they last
+                // (takeGrid), else the arena's next
+                const uint32_t s = splits + j, p = taken0 + s;
+                uint32_t grid;
+                if (p < pool) {
+                    grid = d.gridPool[pool - 1u - p];
+                } else {
+                    const uint32_t first = taken0 < pool ? pool - taken0 : 0u;  // the first split the pool has none for
+                    const unsigned long long off = (unsigned long long)bump0 + (unsigned long long)(s - first) * kGridUnits;
+                    arenaFull |= off + kGridUnits > d.arenaUnits;
+                    grid = off + kGridUnits > d.arenaUnits ? kNone : (uint32_t)off;
+                }
+                const uint32_t node = base + k;
+                d.grid[node] = grid;
+                d.splitIter[node] = batchTag | it;
+                d.dirtyStamp[node] = buildStamp;
+                if (zero0 + s < d.zeroCap) d.zeroList[zero0 + s] = grid;
+                if (dirty0 + s < d.maxNodes) d.dirtyList[dirty0 + s] = node;
+                d.deepPar[j] = k;
+                if (j < kDeepCached / 8u) s_par[j] = k;
             }
             const uint32_t jc = contRun + (pre >> 16);
-            if (wantCont && jc < d.spillingCap) d.spillNodes[jc] = node;
+            if (wantCont && jc < d.spillingCap) d.spillNodes[jc] = base + k;
             want += tot & 0xFFFFu;
             contRun += tot >> 16;
         }
@@ -1338,24 +1344,29 @@ __global__ void __launch_bounds__(1024) k_deep_split(Dev d) {
             break;
         }
         splits += nacc;
-        __syncthreads();  // the split list (deepPar) and the parents' grids are written
+        __syncthreads();  // the split list is written
         // the children of this iteration's splits, ids [hi, hi + 8 nacc)
         for (uint32_t t = threadIdx.x; t < 8u * nacc; t += blockDim.x) {
-            const uint32_t parent = d.deepPar[t >> 3];
-            const uint32_t pm = d.deepMeta[parent - base];
-            makeChild(d, hi + t, parent, t & 7u);
-            const uint32_t meta = (pm & 0xFFFF0000u) | (((pm & 0xFFFFu) << 3) | (t & 7u));
-            d.deepMeta[hi + t - base] = meta;
-            d.deepNode[(size_t)(meta >> 16) * kDeepCells + deepOffset(g + 1u) + (meta & 0xFFFFu)] = hi + t;
+            const uint32_t q = t >> 3;
+            const uint32_t pm = metaAt(q < kDeepCached / 8u ? s_par[q] : d.deepPar[q]);
+            make(hi + t, deepMetaOf(g + 1u, metaSlot(pm), (metaCode(pm) << 3) | (t & 7u)));
         }
         __syncthreads();
         lo = hi;
         hi += 8u * nacc;
     }
+    arenaGrids = taken0 + splits > pool ? taken0 + splits - (taken0 < pool ? pool : taken0) : 0u;
+    if (__syncthreads_or(arenaFull) && threadIdx.x == 0) atomicOr(&c->overflowFlags, (uint32_t)kOvfArena);
     if (threadIdx.x == 0) {
-        c->numNodes = hi;
+        c->numNodes = base + hi;
         c->nodesSplit += splits;
         c->iter = itEnd;
+        c->numZero = zero0 + splits;
+        c->numDirty = dirty0 + splits;
+        c->numGrids += splits;
+        if (pool) c->gridPoolTaken = taken0 + splits;
+        c->arenaBump = bump0 + arenaGrids * kGridUnits;
+        c->refOffset += (unsigned long long)arenaGrids * refAllocSize(kGridBytes);
         if (cont > d.spillingCap) {
             atomicOr(&c->overflowFlags, (uint32_t)kOvfSpilling);
             cont = d.spillingCap;
@@ -1364,7 +1375,66 @@ __global__ void __launch_bounds__(1024) k_deep_split(Dev d) {
     }
 }
 
-// Every point the round moved -- batch points and spilled points whose leaf
+// Everything of the round's node `node` that its record, its root and the
+// round's node table give (doSplitting's child set-up, remolod_octree.cu:323-347):
+// its place, its ancestor row, its children (a node that split in the round;
+// k_deep_split has set its stamps and grid), zero counts and sums. One warp.
+__device__ __forceinline__ void initDeepNode(const Dev& d, uint32_t node, uint32_t meta, uint32_t levels) {
+    const uint32_t lane = laneId();
+    const uint32_t depth = metaDepth(meta), slot = metaSlot(meta), code = metaCode(meta);
+    const uint32_t root = d.splitRecs[slot].node;
+    const uint32_t rootLv = d.level[root];
+    const uint32_t* table = d.deepNode + (size_t)slot * kDeepCells;
+    // lane j < depth: the ancestor j levels below the root
+    const uint32_t anc = lane == 0u ? root : (lane < depth ? table[deepOffset(lane) + (code >> (3u * (depth - lane)))] : kNone);
+    const uint2 link = make_uint2(anc, anc != kNone ? d.grid[anc] : kNone);
+    uint2* row = d.anc + (size_t)node * kMaxDepth;
+    if (lane < rootLv) row[lane] = d.anc[(size_t)root * kMaxDepth + lane];
+    if (lane < depth) row[rootLv + lane] = link;
+    if (lane == depth - 1u) d.parent[node] = link;
+    int32_t kid = -1;
+    if (lane < 8u && depth < levels) kid = (int32_t)table[deepOffset(depth + 1u) + (code << 3) + lane];
+    if (lane < 8u) {
+        d.child[node * 8u + lane] = kid;
+        d.hist8[(size_t)node * 8u + lane] = 0;
+    }
+    const bool split = __any_sync(0xFFFFFFFFu, kid >= 0);
+    if (lane < sizeof(AccumI) / 8u) reinterpret_cast<unsigned long long*>(&d.accum[node])[lane] = 0ull;
+    if (lane == 0u) {
+        uint32_t x = d.nodeX[root], y = d.nodeY[root], z = d.nodeZ[root];
+        for (uint32_t j = depth; j-- > 0u;) {
+            const uint32_t o = code >> (3u * j);
+            x = 2u * x + ((o >> 2) & 1u);
+            y = 2u * y + ((o >> 1) & 1u);
+            z = 2u * z + (o & 1u);
+        }
+        d.level[node] = rootLv + depth;
+        d.nodeX[node] = x;
+        d.nodeY[node] = y;
+        d.nodeZ[node] = z;
+    }
+    if (lane == 1u) {
+        d.numPoints[node] = 0;
+        d.numPointChunks[node] = 0;
+        d.ptTableOff[node] = kNone;
+        d.ptTableCap[node] = 0;
+    }
+    if (lane == 2u) {
+        d.numVoxels[node] = 0;
+        d.numVoxelsStored[node] = 0;
+        d.numVoxelChunks[node] = 0;
+        d.vxTableOff[node] = kNone;
+        d.vxTableCap[node] = 0;
+    }
+    if (lane == 3u && !split) {
+        d.grid[node] = kNone;
+        d.splitIter[node] = 0;
+        d.dirtyStamp[node] = 0;
+    }
+}
+
+// The round's new nodes written whole (initDeepNode), then every point the round
+// moved -- batch points and spilled points whose leaf
 // is a root -- to its leaf in the finished subtree: the deepest node the round
 // made along the point's cube path (k_deep_bin's code), read from the round's
 // node table at every depth at once instead of walking down from the root.
@@ -1375,6 +1445,14 @@ __global__ void __launch_bounds__(256) k_deep_move(Dev d, const Point* __restric
     const uint32_t stamp = c->deepStamp, levels = c->deepLevels;
     const uint32_t ns = c->numSpilled < d.spillCap ? c->numSpilled : d.spillCap;
     const uint32_t total = n + ns;
+    // first the round's new nodes, a warp each, and the roots' new children
+    const uint32_t made = c->numNodes - c->deepBase;
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < made; k += warps) {
+        initDeepNode(d, c->deepBase + k, d.deepMeta[k], levels);
+        if (k < c->deepRoots && laneId() < 8u)
+            d.child[d.splitRecs[k].node * 8u + laneId()] = (int32_t)d.deepNode[(size_t)k * kDeepCells + laneId()];
+    }
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const bool batchPt = i < n;
         uint32_t cur = batchPt ? d.leafOf[i] : d.spillLeaf[i - n];
