@@ -225,6 +225,7 @@ __global__ void __launch_bounds__(kAccumThreads, 3) k_accumulate(Dev d, uint32_t
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t ppc = d.ppc, parts = c->accumParts, step = itemStep(d, parts);
     const unsigned long long bound = c->mortonBound;
+    if (batchIndex == kAtCursor) batchIndex = c->batchletIndex;
     if (threadIdx.x == 0) s_morton = 0ull;
     __syncthreads();
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;

@@ -115,6 +115,7 @@ __global__ void __launch_bounds__(kRollThreads) k_roll(Dev d, RollSum* roll, uin
     unsigned long long(*words)[kRollWords] = s_words[threadIdx.x >> 3];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *ac = AnalysisCounters{};
+        ac->numNodes = nn;
         if (leafA(d, 0)) roll[0] = leafSums(d.accum[0]);  // its origin is the root's
     }
     // the words this lane adds up: lanes 0..5 a 128-bit sum of s2 and one of
@@ -515,7 +516,7 @@ __global__ void __launch_bounds__(256) k_queue_collect(const Dev d, const unsign
 // One block: descending bitonic sort of the candidates in shared memory; the
 // first K become the queue (node ids).
 __global__ void __launch_bounds__(1024) k_queue_sort(const unsigned long long* cand, uint32_t cap, uint32_t K,
-                                                     uint32_t* queue, AnalysisCounters* ac) {
+                                                     uint32_t* queue, AnalysisCounters* ac, AnalysisCounters* host) {
     extern __shared__ unsigned long long s_k[];
     uint32_t n = ac->numCandidates;
     if (n > cap) {
@@ -545,16 +546,29 @@ __global__ void __launch_bounds__(1024) k_queue_sort(const unsigned long long* c
     const uint32_t q = n < K ? n : K;
     for (uint32_t i = threadIdx.x; i < q; i += blockDim.x)
         queue[i] = 0xFFFFFFFFu - (uint32_t)(s_k[i] & 0xFFFFFFFFull);
-    if (threadIdx.x == 0) ac->queueLength = q;
+    // the call's counters, complete now, into the host's pinned copy
+    if (threadIdx.x == 0) {
+        ac->queueLength = q;
+        *host = *ac;
+    }
 }
 
 // Refinement's budgeted pass: the first `budget` queue entries become forced
-// splits of the LOD cut (rb_render's force-large mask).
-__global__ void __launch_bounds__(256) k_refine_mask(const Dev d, uint8_t* mask) {
+// splits of the LOD cut (rb_render's force-large mask). The queue is in
+// descending key order and keys differ, so its prefix is the nodes whose key is
+// at least the last taken entry's: one pass over the nodes writes the mask (a
+// node made since Analysis has no key).
+__global__ void __launch_bounds__(256) k_refine_mask(const Dev d, const uint32_t* queue, const unsigned long long* keys,
+                                                     const AnalysisCounters* ac, uint32_t budget, uint8_t* mask) {
     const uint32_t nn = d.ctr->numNodes;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) mask[i] = 0;
+    const uint32_t q = ac->queueLength < budget ? ac->queueLength : budget;
+    const unsigned long long last = q ? keys[queue[q - 1u]] : ~0ull;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x)
+        mask[i] = i < ac->numNodes && keys[i] >= last ? 1 : 0;
 }
 
+// The same after a queue whose candidates overflowed its sort (it then holds
+// the highest of those that were kept): entry by entry, over a cleared mask.
 __global__ void __launch_bounds__(256) k_refine_set(const uint32_t* queue, const AnalysisCounters* ac,
                                                     uint32_t budget, uint8_t* mask) {
     const uint32_t q = ac->queueLength < budget ? ac->queueLength : budget;
@@ -573,17 +587,18 @@ void launchScore(const Dev& d, NodeAnalysis* out, const float* predictions, unsi
     k_score<<<grid, 256, 0, s>>>(d, out, predictions, keys, hist, p, ac);
 }
 void launchQueue(const Dev& d, const unsigned long long* keys, uint32_t* hist, unsigned long long* cand,
-                 uint32_t candCap, uint32_t K, uint32_t* queue, AnalysisCounters* ac, int grid, cudaStream_t s) {
+                 uint32_t candCap, uint32_t K, uint32_t* queue, AnalysisCounters* ac, AnalysisCounters* host, int grid,
+                 cudaStream_t s) {
     k_queue_threshold<<<1, 1024, 0, s>>>(hist, K, ac);
     k_queue_collect<<<grid, 256, 0, s>>>(d, keys, cand, candCap, hist, ac);
     uint32_t m = 1;
     while (m < candCap) m <<= 1;
-    k_queue_sort<<<1, 1024, (size_t)m * 8, s>>>(cand, candCap, K, queue, ac);
+    k_queue_sort<<<1, 1024, (size_t)m * 8, s>>>(cand, candCap, K, queue, ac, host);
 }
-void launchRefineMask(const Dev& d, const uint32_t* queue, const AnalysisCounters* ac, uint32_t budget,
-                      uint8_t* mask, int grid, cudaStream_t s) {
-    k_refine_mask<<<grid, 256, 0, s>>>(d, mask);
-    k_refine_set<<<grid, 256, 0, s>>>(queue, ac, budget, mask);
+void launchRefineMask(const Dev& d, const uint32_t* queue, const unsigned long long* keys, const AnalysisCounters* ac,
+                      uint32_t budget, bool overflowed, uint8_t* mask, int grid, cudaStream_t s) {
+    k_refine_mask<<<grid, 256, 0, s>>>(d, queue, keys, ac, overflowed ? 0u : budget, mask);
+    if (overflowed) k_refine_set<<<grid, 256, 0, s>>>(queue, ac, budget, mask);
 }
 cudaError_t configureQueueSort(uint32_t candCap) {
     uint32_t m = 1;

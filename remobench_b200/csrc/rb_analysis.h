@@ -66,7 +66,8 @@ struct AnalysisCounters {
     uint32_t numCandidates;
     uint32_t queueLength;
     uint32_t overflow;
-    uint32_t pad[2];
+    uint32_t numNodes;       // nodes the call scored
+    uint32_t pad;
 };
 
 // Every node's sums from the root's origin (launchAnalyze takes them to the
@@ -79,10 +80,12 @@ void launchAnalyze(const Dev& d, RollSum* roll, NodeAnalysis* out, float* featur
 // bins, zero between calls); predictions (2 per node) are read in kScoreLearned mode.
 void launchScore(const Dev& d, NodeAnalysis* out, const float* predictions, unsigned long long* keys, uint32_t* hist,
                  const AnalysisParams& p, AnalysisCounters* ac, int grid, cudaStream_t s);
+// host (pinned) receives the counters once they are complete.
 void launchQueue(const Dev& d, const unsigned long long* keys, uint32_t* hist, unsigned long long* cand,
-                 uint32_t candCap, uint32_t K, uint32_t* queue, AnalysisCounters* ac, int grid, cudaStream_t s);
-void launchRefineMask(const Dev& d, const uint32_t* queue, const AnalysisCounters* ac, uint32_t budget,
-                      uint8_t* mask, int grid, cudaStream_t s);
+                 uint32_t candCap, uint32_t K, uint32_t* queue, AnalysisCounters* ac, AnalysisCounters* host, int grid,
+                 cudaStream_t s);
+void launchRefineMask(const Dev& d, const uint32_t* queue, const unsigned long long* keys, const AnalysisCounters* ac,
+                      uint32_t budget, bool overflowed, uint8_t* mask, int grid, cudaStream_t s);
 cudaError_t configureQueueSort(uint32_t candCap);
 
 }  // namespace rb

@@ -128,7 +128,9 @@ struct rb_ctx {
     // device-driven batches: one graph per batch, the ring descriptor it reads
     cudaGraphExec_t batchGraph = nullptr;
     bool graphTried = false;
-    rb::RingDesc* hostRing = nullptr;  // pinned staging for d.ring
+    // hostCtr holds the device's counters, and the stream has nothing left that
+    // changes the tree: a read-back of it needs no round trip first
+    bool ctrFresh = false;
     // host-ingest ring
     rb::Point* ingestRing = nullptr;
     uint32_t ingestSlots = 0;
@@ -204,10 +206,24 @@ int pointGrid(const rb_ctx* c, uint64_t n) {
 rb_status readCounters(rb_ctx* c) {
     RB_CUDA(c, cudaMemcpyAsync(c->hostCtr, c->d.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, c->stream));
     RB_CUDA(c, cudaStreamSynchronize(c->stream));
+    c->ctrFresh = true;
     return RB_OK;
 }
 
-__global__ void k_build_begin(Counters* c) {
+// The counters for a read-back of the tree: read again only after something
+// may have changed them (ctrFresh).
+rb_status treeCounters(rb_ctx* c) { return c->ctrFresh ? RB_OK : readCounters(c); }
+
+// Starts a build call: its dirty list and clock, and, for device-driven batches
+// (ring != nullptr), the ring they find themselves in, handed over as a kernel
+// parameter instead of a copy ahead of it.
+__global__ void k_build_begin(Counters* c, rb::RingDesc* ring, const __grid_constant__ rb::RingDesc from) {
+    if (ring) {
+        const uint32_t* s = reinterpret_cast<const uint32_t*>(&from);
+        for (uint32_t i = threadIdx.x; i < sizeof(rb::RingDesc) / 4u; i += blockDim.x)
+            reinterpret_cast<uint32_t*>(ring)[i] = s[i];
+    }
+    if (threadIdx.x != 0) return;
     c->buildStamp += 1;
     c->numDirty = 0;
     c->callBatches = 0;
@@ -317,11 +333,7 @@ rb_status checkSync(rb_ctx* c) {
     return RB_OK;
 }
 
-rb_status uploadRing(rb_ctx* c) {
-    RB_CUDA(c, cudaMemcpyAsync(c->d.ring, c->hostRing, sizeof(rb::RingDesc), cudaMemcpyHostToDevice, c->stream));
-    return RB_OK;
-}
-
+// batchIndex rb::kAtCursor: the batches consumed so far, read on the device.
 rb_status accumulate(rb_ctx* c, uint32_t batchIndex) {
     const Dev& d = c->d;
     LAUNCH(c, K_ACCUMULATE, 0, rb::launchAccumulate(d, batchIndex, c->accumAll ? 0 : 1, c->numSMs * 8, c->stream));
@@ -416,8 +428,7 @@ void rb_release(rb_ctx* c) {
     if (c->batchGraph) cudaGraphExecDestroy(c->batchGraph);
     c->batchGraph = nullptr;
     c->graphTried = false;
-    if (c->hostRing) cudaFreeHost(c->hostRing);
-    c->hostRing = nullptr;
+    c->ctrFresh = false;
     c->analyzed = false;
     c->mlp = rb::MlpState{};
     c->mlpReady = false;
@@ -452,6 +463,7 @@ const char* rb_last_error(const rb_ctx* c) { return c ? c->err.c_str() : "null c
 
 rb_status rb_set_stream(rb_ctx* c, void* stream) {
     if (!c) return RB_ERR_INVALID_ARG;
+    c->ctrFresh = false;
     if (c->ownStream && c->stream) cudaStreamDestroy(c->stream);
     c->stream = static_cast<cudaStream_t>(stream);
     c->ownStream = false;
@@ -662,8 +674,6 @@ rb_status rb_allocate(rb_ctx* c, const rb_cloud_meta* meta, uint64_t budget) {
     RB_CUDA(c, cudaMallocHost(&c->hostAccum, sizeof(rb::AccumGlobals)));
     RB_CUDA(c, cudaMallocHost(&c->hostRs, sizeof(rb::RenderResult)));
     RB_CUDA(c, cudaMallocHost(&c->hostActr, sizeof(rb::AnalysisCounters)));
-    RB_CUDA(c, cudaMallocHost(&c->hostRing, sizeof(rb::RingDesc)));
-    std::memset(c->hostRing, 0, sizeof(rb::RingDesc));
     RB_CUDA(c, cudaMemsetAsync(d.ring, 0, sizeof(rb::RingDesc), c->stream));
     RB_CUDA(c, rb::configureQueueSort(kQueueSortCap));
     RB_CUDA(c, rb::configureMlp());
@@ -685,9 +695,7 @@ rb_status rb_reset(rb_ctx* c) {
     if (c->cfg.pipeline == RB_PIPELINE_FLAT) return RB_OK;
     RB_CUDA(c, cudaSetDevice(c->device));
     LAUNCH(c, K_RESET_ROOT, 1, rb::launchResetRoot(c->d, c->numSMs * 2, c->stream));
-    RB_CUDA(c, cudaMemsetAsync(c->d.accumGlobals, 0, sizeof(rb::AccumGlobals), c->stream));
     RB_CUDA(c, cudaGetLastError());
-    RB_CUDA(c, cudaStreamSynchronize(c->stream));
     c->batchesConsumed = 0;
     c->accumAll = true;
     return readCounters(c);  // the host mirror starts from the reset counters
@@ -702,32 +710,32 @@ static rb_status buildFrom(rb_ctx* c, const rb::Point* ring, const uint32_t* siz
     for (uint32_t i = 0; i < std::min(slots, numUploaded); i++)
         if (sizes[i] > slotCap) return fail(c, RB_ERR_CAPACITY, "batch larger than its ring slot");
     const bool graphs = graphPath(c);
+    rb::RingDesc r{};
     if (graphs) {
         if (slots > rb::kMaxRingSlots) return fail(c, RB_ERR_CAPACITY, "more ring slots than a device build handles");
-        rb::RingDesc& r = *c->hostRing;
         r.base = reinterpret_cast<unsigned long long>(ring);
         r.slotCap = slotCap;
         r.numSlots = slots;
         r.numUploaded = numUploaded;
-        r.streamMode = 0;
-        r.first = 0;
-        r.batchSize = 0;
-        r.total = 0;
         r.budgetNs = c->cfg.time_budget_ms > 0.0f ? (unsigned long long)(c->cfg.time_budget_ms * 1e6) : 0ull;
         for (uint32_t i = 0; i < slots; i++) r.sizes[i] = sizes[i];
-        rb_status st = uploadRing(c);
-        if (st != RB_OK) return st;
     }
+    c->ctrFresh = false;
     RB_CUDA(c, cudaEventRecord(c->evStart, c->stream));
-    LAUNCH(c, K_BUILD_BEGIN, 1, (k_build_begin<<<1, 1, 0, c->stream>>>(c->d.ctr)));
+    LAUNCH(c, K_BUILD_BEGIN, 1, (k_build_begin<<<1, 128, 0, c->stream>>>(c->d.ctr, graphs ? c->d.ring : nullptr, r)));
     uint32_t done = 0;
     bool stopped = false;
+    const bool accumOn = c->cfg.accumulate && c->cfg.pipeline == RB_PIPELINE_REMOLOD;
     if (graphs) {
+        // the batches, the fold and the counters' read-back in one run: the host
+        // waits once
         const uint32_t condBefore = c->hostCtr->condRuns;
         const uint64_t pointsBefore = c->hostCtr->numPointsProcessed;
         for (uint32_t k = 0; k < nb; k++) RB_CUDA(c, cudaGraphLaunch(c->batchGraph, c->stream));
-        rb_status st = readCounters(c);
-        if (st != RB_OK) return st;
+        rb_status st = RB_OK;
+        if (accumOn && (st = accumulate(c, rb::kAtCursor)) != RB_OK) return st;
+        RB_CUDA(c, cudaEventRecord(c->evStop, c->stream));
+        if ((st = readCounters(c)) != RB_OK) return st;
         if ((st = checkSync(c)) != RB_OK) return st;
         done = c->hostCtr->batchletIndex - first;
         stopped = c->hostCtr->batchStop && c->hostCtr->stopReason == rb::kStopMemory;
@@ -745,14 +753,16 @@ static rb_status buildFrom(rb_ctx* c, const rb::Point* ring, const uint32_t* siz
         if (c->cfg.time_budget_ms > 0.0f && ms > c->cfg.time_budget_ms) break;
     }
     c->batchesConsumed = first + done;
-    if (c->cfg.accumulate && c->cfg.pipeline == RB_PIPELINE_REMOLOD) {
-        rb_status st = accumulate(c, c->batchesConsumed);
-        if (st != RB_OK) return st;
-    } else if (done > 0) {
-        c->accumAll = true;
+    if (!graphs) {
+        if (accumOn) {
+            rb_status st = accumulate(c, c->batchesConsumed);
+            if (st != RB_OK) return st;
+        }
+        c->ctrFresh = false;  // read between a batch's launches
+        RB_CUDA(c, cudaEventRecord(c->evStop, c->stream));
+        RB_CUDA(c, cudaEventSynchronize(c->evStop));
     }
-    RB_CUDA(c, cudaEventRecord(c->evStop, c->stream));
-    RB_CUDA(c, cudaEventSynchronize(c->evStop));
+    if (!accumOn && done > 0) c->accumAll = true;
     if (out) {
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, c->evStart, c->evStop);
@@ -805,8 +815,8 @@ rb_status rb_ingest_host(rb_ctx* c, const rb_point* points, uint64_t n, uint32_t
     const bool graphs = graphPath(c);
     uint64_t pointsBefore = 0;
     uint32_t condBefore = 0;
+    rb::RingDesc r{};
     if (graphs) {
-        rb::RingDesc& r = *c->hostRing;
         r.base = reinterpret_cast<unsigned long long>(c->ingestRing);
         r.slotCap = c->cfg.slot_capacity;
         r.numSlots = S;
@@ -815,14 +825,12 @@ rb_status rb_ingest_host(rb_ctx* c, const rb_point* points, uint64_t n, uint32_t
         r.first = firstBatch;
         r.batchSize = batchSize;
         r.total = n;
-        r.budgetNs = 0;
-        rb_status st = uploadRing(c);
-        if (st != RB_OK) return st;
         condBefore = c->hostCtr->condRuns;
         pointsBefore = c->hostCtr->numPointsProcessed;
     }
+    c->ctrFresh = false;
     RB_CUDA(c, cudaEventRecord(c->evStart, c->stream));
-    LAUNCH(c, K_BUILD_BEGIN, 1, (k_build_begin<<<1, 1, 0, c->stream>>>(c->d.ctr)));
+    LAUNCH(c, K_BUILD_BEGIN, 1, (k_build_begin<<<1, 128, 0, c->stream>>>(c->d.ctr, graphs ? c->d.ring : nullptr, r)));
     // the copy stream fills slot (b % S) once the compute stream released it
     auto issueCopy = [&](uint64_t b) -> rb_status {
         const uint32_t slot = (uint32_t)(b % S);
@@ -883,6 +891,7 @@ rb_status rb_ingest_host(rb_ctx* c, const rb_point* points, uint64_t n, uint32_t
     RB_CUDA(c, cudaEventRecord(c->evStop, c->stream));
     RB_CUDA(c, cudaEventSynchronize(c->evStop));
     RB_CUDA(c, cudaStreamSynchronize(c->copyStream));
+    c->ctrFresh = false;
     if (graphs) {
         rb_status st = readCounters(c);
         if (st != RB_OK) return st;
@@ -907,6 +916,7 @@ rb_status rb_accumulate(rb_ctx* c, uint32_t batchIndex, rb_accum_globals* out) {
     if (!c) return RB_ERR_INVALID_ARG;
     if (!c->allocated || c->cfg.pipeline == RB_PIPELINE_FLAT) return fail(c, RB_ERR_STATE, "no tree");
     RB_CUDA(c, cudaSetDevice(c->device));
+    c->ctrFresh = false;
     rb_status st = accumulate(c, batchIndex);
     if (st != RB_OK) return st;
     if (out) {
@@ -1066,7 +1076,7 @@ rb_status rb_read_nodes(rb_ctx* c, rb_node_info* out, uint32_t capacity, uint32_
     if (!c || !count) return RB_ERR_INVALID_ARG;
     if (!c->allocated || c->cfg.pipeline == RB_PIPELINE_FLAT) return fail(c, RB_ERR_STATE, "no tree");
     RB_CUDA(c, cudaSetDevice(c->device));
-    rb_status st = readCounters(c);
+    rb_status st = treeCounters(c);
     if (st != RB_OK) return st;
     const uint32_t nn = c->hostCtr->numNodes;
     *count = nn;
@@ -1195,10 +1205,9 @@ rb_status rb_analyze(rb_ctx* c, const rb_frame* f, const rb_analysis_params* p, 
     LAUNCH(c, K_SCORE, 0, rb::launchScore(c->d, c->analysis, c->predictions, c->akeys, c->ahist, ap, c->actr, grid,
                                           s));
     LAUNCH(c, K_QUEUE, 0, rb::launchQueue(c->d, c->akeys, c->ahist, c->acand, kQueueSortCap, p->queue_capacity,
-                                          c->aqueue, c->actr, grid, s));
+                                          c->aqueue, c->actr, c->hostActr, grid, s));
     RB_CUDA(c, cudaGetLastError());
     RB_CUDA(c, cudaEventRecord(c->evStop, s));
-    RB_CUDA(c, cudaMemcpyAsync(c->hostActr, c->actr, sizeof(rb::AnalysisCounters), cudaMemcpyDeviceToHost, s));
     RB_CUDA(c, cudaStreamSynchronize(s));
     c->analyzed = true;
     if (out) {
@@ -1228,7 +1237,7 @@ rb_status rb_read_analysis(rb_ctx* c, rb_node_analysis* out, uint32_t capacity, 
     if (!c->analyzed) return fail(c, RB_ERR_STATE, "read before rb_analyze");
     static_assert(sizeof(rb_node_analysis) == sizeof(rb::NodeAnalysis), "analysis layout");
     RB_CUDA(c, cudaSetDevice(c->device));
-    rb_status st = readCounters(c);
+    rb_status st = treeCounters(c);
     if (st != RB_OK) return st;
     return copyOut(c, out, c->analysis, sizeof(rb_node_analysis), capacity, count, c->hostCtr->numNodes);
 }
@@ -1237,7 +1246,7 @@ rb_status rb_read_features(rb_ctx* c, float* out, uint32_t capacity, uint32_t* c
     if (!c || !count) return RB_ERR_INVALID_ARG;
     if (!c->analyzed) return fail(c, RB_ERR_STATE, "read before rb_analyze");
     RB_CUDA(c, cudaSetDevice(c->device));
-    rb_status st = readCounters(c);
+    rb_status st = treeCounters(c);
     if (st != RB_OK) return st;
     return copyOut(c, out, c->features, sizeof(float) * rb::kIn, capacity, count, c->hostCtr->numNodes);
 }
@@ -1381,7 +1390,7 @@ rb_status rb_read_rollup(rb_ctx* c, uint64_t* out16, uint32_t capacity, uint32_t
     if (!c || !count) return RB_ERR_INVALID_ARG;
     if (!c->analyzed) return fail(c, RB_ERR_STATE, "read before rb_analyze");
     RB_CUDA(c, cudaSetDevice(c->device));
-    rb_status st = readCounters(c);
+    rb_status st = treeCounters(c);
     if (st != RB_OK) return st;
     const uint32_t nn = c->hostCtr->numNodes;
     *count = nn;
@@ -1402,8 +1411,9 @@ rb_status rb_refine(rb_ctx* c, uint32_t budget, uint64_t maskDev) {
     if (!c || !maskDev) return RB_ERR_INVALID_ARG;
     if (!c->analyzed) return fail(c, RB_ERR_STATE, "refine before rb_analyze");
     RB_CUDA(c, cudaSetDevice(c->device));
-    LAUNCH(c, K_REFINE, budget, rb::launchRefineMask(c->d, c->aqueue, c->actr, budget,
-                                                     reinterpret_cast<uint8_t*>(maskDev), c->numSMs * 2, c->stream));
+    LAUNCH(c, K_REFINE, budget,
+           rb::launchRefineMask(c->d, c->aqueue, c->akeys, c->actr, budget, c->hostActr->overflow != 0u,
+                                reinterpret_cast<uint8_t*>(maskDev), c->numSMs * 2, c->stream));
     RB_CUDA(c, cudaGetLastError());
     RB_CUDA(c, cudaStreamSynchronize(c->stream));
     return RB_OK;
@@ -1448,6 +1458,7 @@ rb_status rb_refine_deepen(rb_ctx* c, uint32_t budget, uint32_t min_points, rb_d
     if (st != RB_OK) return st;
     if ((st = readCounters(c)) != RB_OK) return st;
     const rb::Counters& k = *c->hostCtr;
+    c->ctrFresh = false;
     // the queue names nodes by their role before the pass
     c->analyzed = false;
     if (out) {
@@ -1486,6 +1497,7 @@ rb_status rb_refine_collapse(rb_ctx* c, const uint32_t* nodes, uint32_t count, u
     RB_CUDA(c, cudaGetLastError());
     if ((st = readCounters(c)) != RB_OK) return st;
     const rb::Counters& k = *c->hostCtr;
+    c->ctrFresh = false;
     c->analyzed = false;
     if (out) {
         out->nodes_collapsed = k.collapseSelected;
@@ -1541,7 +1553,7 @@ rb_status rb_read_accums(rb_ctx* c, rb_accum* out, uint32_t capacity, uint32_t* 
     if (!c->allocated || c->cfg.pipeline == RB_PIPELINE_FLAT) return fail(c, RB_ERR_STATE, "no tree");
     static_assert(sizeof(rb_accum) == sizeof(rb::AccumI), "accumulator layout");
     RB_CUDA(c, cudaSetDevice(c->device));
-    rb_status st = readCounters(c);
+    rb_status st = treeCounters(c);
     if (st != RB_OK) return st;
     const uint32_t nn = c->hostCtr->numNodes;
     *count = nn;

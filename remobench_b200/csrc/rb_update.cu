@@ -2833,6 +2833,7 @@ __global__ void k_reset_root(Dev d) {
         d.dirtyStamp[0] = 0;
         AccumI za = {};
         d.accum[0] = za;
+        *d.accumGlobals = AccumGlobals{};
         c->arenaBump = kGridUnits;
         c->numGrids = 1;
         c->refOffset += refAllocSize(kGridBytes);

@@ -65,3 +65,72 @@ def test_queue_is_the_top_k(c1_cloud, k):
         assert r.overflow == 0 and np.array_equal(q, order[:k])
         r = ctx.analyze(f, frontier_only=False, queue_capacity=k)
     ctx.close()
+
+
+def test_mask_is_the_queue_prefix_on_a_changed_tree(c1_cloud):
+    """The mask marks the queue's prefix, and nothing else: after an analysis of
+    a larger tree whose keys are still there, and when the tree grew since."""
+    import torch
+    from remobench_b200.lod import Context, DeviceRing, make_frame
+    _, cloud, bmin, bmax = c1_cloud
+    cloud = np.ascontiguousarray(cloud[:400_000])
+    f = make_frame(bmin, bmax, 1920, 1080, yaw=1.2, pitch=-0.5, radius_scale=0.5)
+    ctx = Context(slot_capacity=100_000, max_points_per_node=1000, time_budget_ms=0.0, max_batches_per_build=1,
+                  store_capacity=4 << 30)
+    ctx.allocate(len(cloud), bmin, bmax)
+    ring = DeviceRing(cloud, 100_000, slots=ctx.cfg.ring_slots, slot_capacity=100_000)
+    ring.upload_window(0)
+    mask = torch.empty(ctx.cfg.max_nodes, dtype=torch.uint8, device="cuda")
+    for upto in (4, 1):  # a large tree first, then a small one after a reset
+        ctx.reset()
+        for k in range(upto):
+            ctx.build(ring.ring, ring.sizes, k + 1, ring.num_batches)
+        ctx.analyze(f, frontier_only=False, queue_capacity=2000)
+        q = ctx.queue()
+        for grown in (False, True):
+            if grown:
+                ctx.build(ring.ring, ring.sizes, min(upto + 1, 4), ring.num_batches)
+            nn = ctx.stats().num_nodes
+            for budget in (0, 1, len(q) // 2, len(q), 1 << 30):
+                mask.fill_(7)
+                torch.cuda.synchronize()
+                ctx.refine(budget, mask)
+                m = mask.cpu().numpy()
+                assert set(np.nonzero(m[:nn])[0].tolist()) == set(q[:budget].tolist())
+                assert np.all(m[:nn] <= 1) and np.all(m[nn:] == 7)
+    ctx.close()
+
+
+def test_read_backs_follow_every_change(c1_cloud):
+    """Nodes, sums and analysis read right after each call that changes the tree."""
+    from remobench_b200.lod import Context, DeviceRing, make_frame
+    _, cloud, bmin, bmax = c1_cloud
+    cloud = np.ascontiguousarray(cloud[:400_000])
+    f = make_frame(bmin, bmax, 1920, 1080, yaw=1.2, pitch=-0.5, radius_scale=0.5)
+    for graphs in (1, 0):
+        ctx = Context(slot_capacity=100_000, max_points_per_node=5000, time_budget_ms=0.0, max_batches_per_build=1,
+                      use_graphs=graphs)
+        ctx.allocate(len(cloud), bmin, bmax)
+        ring = DeviceRing(cloud, 100_000, slots=ctx.cfg.ring_slots, slot_capacity=100_000)
+        ring.upload_window(0)
+        assert len(ctx.nodes()) == 1
+        for k in range(4):
+            r = ctx.build(ring.ring, ring.sizes, k + 1, ring.num_batches)
+            assert r.batches_this_call == 1 and r.batches_consumed == k + 1
+            nodes, sums = ctx.nodes(), ctx.accums()
+            assert len(nodes) == len(sums) == ctx.stats().num_nodes
+            assert int(sums["count"].sum()) == int(nodes["num_points"][nodes["is_leaf"] == 1].sum()) == 100_000 * (k + 1)
+            assert np.all(sums["last_touched_batch"][sums["count"] > 0] <= k + 1)
+            assert np.any(sums["last_touched_batch"] == k + 1)
+        ctx.analyze(f, frontier_only=False)
+        before = len(ctx.nodes())
+        assert len(ctx.analysis()) == len(ctx.features()) == before
+        d = ctx.refine_deepen(8)
+        assert len(ctx.nodes()) == before + 8 * d.nodes_split and d.nodes_split > 0
+        assert int(ctx.accums()["count"].sum()) == len(cloud)
+        ctx.reset()
+        assert len(ctx.nodes()) == 1 and int(ctx.accums()["count"].sum()) == 0
+        r = ctx.ingest_host(cloud, 100_000)
+        assert r.batches_consumed == 4 and len(ctx.nodes()) == ctx.stats().num_nodes > 1
+        assert int(ctx.accums()["count"].sum()) == len(cloud)
+        ctx.close()
