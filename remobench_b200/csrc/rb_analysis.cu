@@ -53,8 +53,8 @@ __device__ __forceinline__ bool leafA(const Dev& d, uint32_t node) {
 // by the longest chain of dependent round trips, one arrival and one read per
 // level of the tree, not by bytes (184 B read and written per node). Measured
 // at 31,497 nodes: 232 us as a launch per level (a pass over all nodes for each
-// of the 21, whatever the tree's depth), 40 us so; at 2,000 nodes 120 and
-// 27 us. Re-basing at every step of the chain instead: 59 and 33 us.
+// of the 21, whatever the tree's depth), 37 us so; at 2,000 nodes 120 and
+// 23 us. Re-basing at every step of the chain instead: 59 and 33 us.
 constexpr uint32_t kRollThreads = 128;
 constexpr uint32_t kRollWords = sizeof(RollSum) / 8u;
 
@@ -158,7 +158,9 @@ __global__ void __launch_bounds__(kRollThreads) k_roll(Dev d, RollSum* roll, uin
             }
             __syncwarp(gmask);
             unsigned long long a = 0, b = 0, e = 0, lt = 0;
-#pragma unroll
+            // half unrolled: a climb runs this cold, and eight copies cost more in
+            // instruction fetches than they save (27 against 23 us at 2,000 nodes)
+#pragma unroll 2
             for (uint32_t m = 0; m < 8u; m++) {
                 const unsigned long long va = words[m][w0];
                 a += va;
