@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include "rb_kernels.h"
+#include "rb_launch.h"
 #include "rb_state.h"
 
 namespace rb {
@@ -87,6 +88,7 @@ constexpr unsigned long long kAccumFine = 3000000ull;
 // globals per launch), and how its chunks are cut, from the points that came in
 // since the last one.
 __global__ void k_accum_begin(Dev d) {
+    follow();
     Counters* c = d.ctr;
     AccumGlobals* g = d.accumGlobals;
     g->sumLeafCounts = 0;
@@ -125,6 +127,7 @@ __device__ __forceinline__ unsigned long long mortonCode(uint32_t x, uint32_t y,
 // least its leaf's lower corner's (clamping only raises a coordinate), and the
 // largest lower corner of the leaves with new points bounds it from below.
 __global__ void __launch_bounds__(256) k_accum_plan(Dev d, int useList) {
+    follow();
     __shared__ uint32_t s_warp[8];
     __shared__ uint32_t s_base, s_leaves;
     __shared__ unsigned long long s_points, s_bound;
@@ -219,6 +222,7 @@ __device__ __forceinline__ void add128pair(unsigned long long& lo, unsigned long
 // took 108 us with a division per coordinate, 64-bit clamps and a Morton
 // comparison per point, 77 us without (4.2 TB/s of the points read).
 __global__ void __launch_bounds__(kAccumThreads, 3) k_accumulate(Dev d, uint32_t batchIndex, int useList) {
+    follow();
     __shared__ unsigned long long s_morton;
     const Counters* c = d.ctr;
     const uint32_t items = c->accumItems;
@@ -390,6 +394,7 @@ __global__ void __launch_bounds__(kAccumThreads, 3) k_accumulate(Dev d, uint32_t
 // kernel_accum_verify (remolod_accum.cu:214-233). One thread restarts the dirty
 // list, which names the nodes touched since this fold (nothing here reads it).
 __global__ void __launch_bounds__(256) k_accum_verify(Dev d) {
+    follow();
     const uint32_t nn = d.ctr->numNodes;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         d.ctr->buildStamp += 1u;
@@ -407,9 +412,9 @@ __global__ void __launch_bounds__(256) k_accum_verify(Dev d) {
 
 void launchAccumulate(const Dev& d, uint32_t batchIndex, int useList, int grid, cudaStream_t s) {
     k_accum_begin<<<1, 1, 0, s>>>(d);
-    k_accum_plan<<<grid / 4 + 1, 256, 0, s>>>(d, useList);
-    k_accumulate<<<grid, kAccumThreads, 0, s>>>(d, batchIndex, useList);
+    launchBehind(k_accum_plan, grid / 4 + 1, 256, 0, s, d, useList);
+    launchBehind(k_accumulate, grid, kAccumThreads, 0, s, d, batchIndex, useList);
 }
-void launchAccumVerify(const Dev& d, int grid, cudaStream_t s) { k_accum_verify<<<grid, 256, 0, s>>>(d); }
+void launchAccumVerify(const Dev& d, int grid, cudaStream_t s) { launchBehind(k_accum_verify, grid, 256, 0, s, d); }
 
 }  // namespace rb

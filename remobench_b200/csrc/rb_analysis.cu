@@ -22,6 +22,7 @@
 
 #include "rb_analysis.h"
 #include "rb_kernels.h"
+#include "rb_launch.h"
 #include "rb_state.h"
 
 namespace rb {
@@ -108,6 +109,7 @@ __device__ __forceinline__ uint32_t arriveAcqRel(uint32_t* p) {
 
 __global__ void __launch_bounds__(kRollThreads) k_roll(Dev d, RollSum* roll, uint32_t* rollArrive,
                                                        AnalysisCounters* ac) {
+    follow();
     __shared__ unsigned long long s_words[kRollThreads / 8][8][kRollWords];
     const uint32_t nn = d.ctr->numNodes;
     const uint32_t oct = threadIdx.x & 7u;
@@ -282,6 +284,7 @@ __device__ __forceinline__ F4a mat(const float* m, float x, float y, float z) {
 __global__ void __launch_bounds__(256) k_analyze(Dev d, RollSum* roll, NodeAnalysis* out,
                                                  float* features, AnalysisParams prm, Frame f,
                                                  AnalysisCounters* ac) {
+    follow();
     const uint32_t nn = d.ctr->numNodes;
     const float cube = fmaxf(fmaxf(f.boxMax[0] - f.boxMin[0], f.boxMax[1] - f.boxMin[1]), f.boxMax[2] - f.boxMin[2]);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
@@ -432,6 +435,7 @@ __global__ void __launch_bounds__(256) k_analyze(Dev d, RollSum* roll, NodeAnaly
 // correction (output 0, x 1/300).
 __global__ void __launch_bounds__(256) k_score(Dev d, NodeAnalysis* out, const float* pred, unsigned long long* keys,
                                                uint32_t* hist, AnalysisParams prm, AnalysisCounters* ac) {
+    follow();
     const uint32_t nn = d.ctr->numNodes;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
         NodeAnalysis o = out[i];
@@ -460,6 +464,7 @@ __global__ void __launch_bounds__(256) k_score(Dev d, NodeAnalysis* out, const f
 // a load per bin and a scan by one thread, 21 us with 16 loads a thread at a
 // stride of 256 B, 5 us so.
 __global__ void __launch_bounds__(1024) k_queue_threshold(const uint32_t* hist, uint32_t K, AnalysisCounters* ac) {
+    follow();
     __shared__ uint32_t s_warp[32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     // row j, lane l: bins top - 128 j - 4 l - 3 .. top - 128 j - 4 l
@@ -501,6 +506,7 @@ __global__ void __launch_bounds__(1024) k_queue_threshold(const uint32_t* hist, 
 __global__ void __launch_bounds__(256) k_queue_collect(const Dev d, const unsigned long long* keys,
                                                        unsigned long long* cand, uint32_t cap, uint32_t* hist,
                                                        AnalysisCounters* ac) {
+    follow();
     const uint32_t nn = d.ctr->numNodes;
     const uint32_t thr = ac->thresholdBin;
     // the histogram back to zero for the next call
@@ -519,6 +525,7 @@ __global__ void __launch_bounds__(256) k_queue_collect(const Dev d, const unsign
 // first K become the queue (node ids).
 __global__ void __launch_bounds__(1024) k_queue_sort(const unsigned long long* cand, uint32_t cap, uint32_t K,
                                                      uint32_t* queue, AnalysisCounters* ac, AnalysisCounters* host) {
+    follow();
     extern __shared__ unsigned long long s_k[];
     uint32_t n = ac->numCandidates;
     if (n > cap) {
@@ -582,20 +589,20 @@ void launchRoll(const Dev& d, RollSum* roll, uint32_t* rollArrive, AnalysisCount
 }
 void launchAnalyze(const Dev& d, RollSum* roll, NodeAnalysis* out, float* features,
                    const AnalysisParams& p, const Frame& f, AnalysisCounters* ac, int grid, cudaStream_t s) {
-    k_analyze<<<grid, 256, 0, s>>>(d, roll, out, features, p, f, ac);
+    launchBehind(k_analyze, grid, 256, 0, s, d, roll, out, features, p, f, ac);
 }
 void launchScore(const Dev& d, NodeAnalysis* out, const float* predictions, unsigned long long* keys, uint32_t* hist,
                  const AnalysisParams& p, AnalysisCounters* ac, int grid, cudaStream_t s) {
-    k_score<<<grid, 256, 0, s>>>(d, out, predictions, keys, hist, p, ac);
+    launchBehind(k_score, grid, 256, 0, s, d, out, predictions, keys, hist, p, ac);
 }
 void launchQueue(const Dev& d, const unsigned long long* keys, uint32_t* hist, unsigned long long* cand,
                  uint32_t candCap, uint32_t K, uint32_t* queue, AnalysisCounters* ac, AnalysisCounters* host, int grid,
                  cudaStream_t s) {
-    k_queue_threshold<<<1, 1024, 0, s>>>(hist, K, ac);
-    k_queue_collect<<<grid, 256, 0, s>>>(d, keys, cand, candCap, hist, ac);
+    launchBehind(k_queue_threshold, 1, 1024, 0, s, hist, K, ac);
+    launchBehind(k_queue_collect, grid, 256, 0, s, d, keys, cand, candCap, hist, ac);
     uint32_t m = 1;
     while (m < candCap) m <<= 1;
-    k_queue_sort<<<1, 1024, (size_t)m * 8, s>>>(cand, candCap, K, queue, ac, host);
+    launchBehind(k_queue_sort, 1, 1024, (size_t)m * 8, s, cand, candCap, K, queue, ac, host);
 }
 void launchRefineMask(const Dev& d, const uint32_t* queue, const unsigned long long* keys, const AnalysisCounters* ac,
                       uint32_t budget, bool overflowed, uint8_t* mask, int grid, cudaStream_t s) {

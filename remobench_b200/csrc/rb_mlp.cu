@@ -31,6 +31,7 @@
 #include <cuda_runtime.h>
 
 #include "rb_mlp.h"
+#include "rb_launch.h"
 
 namespace rb {
 
@@ -282,6 +283,7 @@ __device__ __forceinline__ float sumRows(float v) {
 __global__ void __launch_bounds__(kWarps * 32, 2) k_mlp_grad(const __nv_bfloat16* wq, const float* params,
                                                              const float* __restrict__ x,
                                                              const float* __restrict__ tgt, uint32_t n, float* grad) {
+    follow();
     extern __shared__ __align__(16) unsigned char s_raw[];
     SmemWeights& s = *reinterpret_cast<SmemWeights*>(s_raw);
     SmemStage& st = *reinterpret_cast<SmemStage*>(s_raw + sizeof(SmemWeights));
@@ -470,6 +472,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) k_mlp_grad(const __nv_bfloat16
 // and the sum in hostLoss (pinned).
 __global__ void k_mlp_adam(float* params, float* grad, float* m, float* v, __nv_bfloat16* wq, AdamStep a,
                            float* hostLoss) {
+    follow();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kNumParams; i += gridDim.x * blockDim.x) {
         const float g = grad[i];
         grad[i] = 0.0f;
@@ -521,7 +524,7 @@ void launchMlpGrad(const MlpState& st, const float* x, const float* t, uint32_t 
 }
 
 void launchMlpAdam(const MlpState& st, const AdamStep& a, float* hostLoss, cudaStream_t s) {
-    k_mlp_adam<<<(kNumParams + 255) / 256, 256, 0, s>>>(st.params, st.grad, st.m, st.v, st.wq, a, hostLoss);
+    launchBehind(k_mlp_adam, (kNumParams + 255) / 256, 256, 0, s, st.params, st.grad, st.m, st.v, st.wq, a, hostLoss);
 }
 
 void launchMlpQuantize(const MlpState& st, cudaStream_t s) {

@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include "rb_kernels.h"
+#include "rb_launch.h"
 #include "rb_state.h"
 
 namespace rb {
@@ -238,6 +239,7 @@ __device__ __forceinline__ uint32_t storedVoxels(const Dev& d, uint32_t node) {
 __global__ void __launch_bounds__(256) k_cut(Dev d, Frame f, unsigned long long* fb, uint64_t npx,
                                              const uint8_t* forceLarge, RenderScratch* rs, DrawItem* items,
                                              uint32_t cap) {
+    follow();
     __shared__ Plane s_pl[6];
     if (threadIdx.x == 0) {
         Plane pl[6];
@@ -334,6 +336,7 @@ template <bool kOnePixel>
 __global__ void __launch_bounds__(256, 6) k_raster(Dev d, Frame f, unsigned long long* fb,
                                                 const RenderScratch* rs, const DrawItem* items,
                                                 uint32_t cap, RenderResult* host) {
+    follow();
     constexpr uint32_t kDraw = 2;
     const uint32_t ni = listedItems(rs, cap);
     const uint32_t lane = threadIdx.x & 31u;
@@ -528,6 +531,7 @@ constexpr int kEdlW = 64;
 template <int kEdlRows>
 __global__ void __launch_bounds__(256) k_edl(unsigned long long* fb, uint32_t* rgba, uint32_t width, uint32_t height,
                                              float strength) {
+    follow();
     constexpr int kEdlH = 4 * kEdlRows;
     __shared__ float s_log[kEdlH + 2][kEdlW + 2];
     const int w = (int)width, h = (int)height;
@@ -615,8 +619,8 @@ void launchCut(const Dev& d, const Frame& f, unsigned long long* fb, uint64_t np
 }
 void launchRaster(const Dev& d, const Frame& f, unsigned long long* fb, const RenderScratch* rs,
                   const DrawItem* items, uint32_t cap, RenderResult* host, int grid, cudaStream_t s) {
-    if (f.pointSize / 2 == 0) k_raster<true><<<grid, 256, 0, s>>>(d, f, fb, rs, items, cap, host);
-    else k_raster<false><<<grid, 256, 0, s>>>(d, f, fb, rs, items, cap, host);
+    if (f.pointSize / 2 == 0) launchBehind(k_raster<true>, grid, 256, 0, s, d, f, fb, rs, items, cap, host);
+    else launchBehind(k_raster<false>, grid, 256, 0, s, d, f, fb, rs, items, cap, host);
 }
 void launchRasterFlat(const Frame& f, unsigned long long* fb, const Point* pts, uint64_t n, int grid,
                       cudaStream_t s) {
@@ -629,8 +633,8 @@ void launchEdl(unsigned long long* fb, uint32_t* rgba, uint32_t w, uint32_t h, f
     const bool tall = (uint64_t)w * h >= (4ull << 20);
     const uint32_t rows = tall ? 32u : 16u;
     const dim3 grid((w + kEdlW - 1u) / kEdlW, min((h + rows - 1u) / rows, 65535u));
-    if (tall) k_edl<8><<<grid, 256, 0, s>>>(fb, rgba, w, h, strength);
-    else k_edl<4><<<grid, 256, 0, s>>>(fb, rgba, w, h, strength);
+    if (tall) launchBehind(k_edl<8>, grid, 256, 0, s, fb, rgba, w, h, strength);
+    else launchBehind(k_edl<4>, grid, 256, 0, s, fb, rgba, w, h, strength);
 }
 void launchResolve(const unsigned long long* fb, uint32_t* rgba, uint64_t npx, int grid, cudaStream_t s) {
     k_resolve<<<grid, 256, 0, s>>>(fb, rgba, npx);

@@ -15,6 +15,7 @@
 #include <cstring>
 
 #include "rb_kernels.h"
+#include "rb_launch.h"
 #include "rb_state.h"
 
 namespace rb {
@@ -189,6 +190,7 @@ __device__ __forceinline__ uint32_t blockReserve(BlockSlots& b, uint32_t* counte
 __device__ __forceinline__ void resetBatchCounters(Counters* c);
 
 __global__ void k_batch_begin(Dev d, uint32_t fromRing) {
+    follow();
     Counters* c = d.ctr;
     uint32_t reason = 0;
     if (fromRing) {
@@ -259,6 +261,7 @@ __device__ __forceinline__ void resetBatchCounters(Counters* c) {
 
 // Each block takes one contiguous, warp-aligned range of the batch.
 __global__ void __launch_bounds__(256) k_count_first(Dev d, const Point* __restrict__ pts, uint32_t n) {
+    follow();
     __shared__ BlockCounts s_counts;
     if (d.ctr->batchStop) return;
     RB_BATCH_AT_CURSOR(d, pts, n);
@@ -1003,6 +1006,7 @@ __device__ __forceinline__ void deepBookCounters(const Dev& d, Counters* c, uint
 // batch) when no node can be split, more than kDeepRoots spill, or a root
 // lies too deep to bin below.
 __global__ void __launch_bounds__(1024) k_deep_book(Dev d) {
+    follow();
     __shared__ uint32_t s_sort[kDeepRoots];
     __shared__ uint32_t s_warp[32];
     __shared__ uint32_t s_maxLevel;
@@ -1165,6 +1169,7 @@ __device__ __forceinline__ void deepBin(const Dev& d, DeepBlockBins& bins, bool 
 // run of the batch (neighbouring points share cubes). Each is binned below
 // its root.
 __global__ void __launch_bounds__(256) k_deep_bin(Dev d, const Point* __restrict__ pts, uint32_t n) {
+    follow();
     __shared__ DeepBlockBins s_bins;
     const Counters* c = d.ctr;
     if (c->batchStop || !c->deepActive) return;
@@ -1258,6 +1263,7 @@ static_assert(kDeepRoots <= 4096u && 3u * kDeepLevels <= 16u, "deepMeta's fields
 constexpr uint32_t kDeepCached = 4096;  // records and split nodes kept in shared memory
 
 __global__ void __launch_bounds__(1024) k_deep_split(Dev d) {
+    follow();
     __shared__ uint32_t s_warp[32];
     __shared__ uint32_t s_meta[kDeepCached];
     __shared__ uint32_t s_par[kDeepCached / 8u];
@@ -1439,6 +1445,7 @@ __device__ __forceinline__ void initDeepNode(const Dev& d, uint32_t node, uint32
 // made along the point's cube path (k_deep_bin's code), read from the round's
 // node table at every depth at once instead of walking down from the root.
 __global__ void __launch_bounds__(256) k_deep_move(Dev d, const Point* __restrict__ pts, uint32_t n) {
+    follow();
     const Counters* c = d.ctr;
     if (c->batchStop || !c->deepActive) return;
     RB_BATCH_AT_CURSOR(d, pts, n);
@@ -2230,6 +2237,7 @@ __device__ __forceinline__ void blockReserveMany(BlockSlots& b, uint32_t* counte
 // blockDim.x) and issues each step's loads for all of them before using any,
 // so one iteration waits on three rounds of memory instead of three per entry.
 __global__ void __launch_bounds__(256) k_vox_commit(Dev d) {
+    follow();
     __shared__ BlockSlots s_slots;
     const Counters* c = d.ctr;
     if (c->batchStop) return;
@@ -2376,6 +2384,7 @@ __global__ void __launch_bounds__(256) k_alloc_points(Dev d) {
 // allocateVoxelChunks (:885-916), one thread per node, after k_vox_commit
 // has counted the batch's new voxels.
 __global__ void __launch_bounds__(256) k_alloc_voxels(Dev d) {
+    follow();
     Counters* c = d.ctr;
     if (c->batchStop) return;
     const uint32_t nn = c->numNodes;
@@ -2469,6 +2478,7 @@ __global__ void __launch_bounds__(256) k_insert(Dev d, const Point* __restrict__
 // centre (:124-134) with its representative's colour, from the compact lists
 // k_vox_commit made.
 __global__ void __launch_bounds__(256) k_vox_store(Dev d) {
+    follow();
     const Counters* c = d.ctr;
     if (c->batchStop) return;
     const uint32_t nnew = newCellCount(d);
@@ -2928,7 +2938,11 @@ void launchResetRoot(const Dev& d, int grid, cudaStream_t s) { k_reset_root<<<gr
 // own; k_vox_lift, k_vox_commit, k_alloc_voxels, k_vox_store) and the point path
 // (k_alloc_points, k_insert) read the finished tree and write disjoint node
 // fields and chunks, so the point path runs in the voxel path's shadow; they
-// join before k_batch_end. One graph launch builds the batch at batchletIndex
+// join before k_batch_end. A kernel with one kernel before it and little to do
+// itself is launched behind that one (launchBehind): a batch of 250,000 points
+// 101 -> 97 us, of a million 168 -> 165. Behind k_expand_rest, or before the
+// join of the levels branch, it gave nothing more; with that branch on the main
+// stream the batches of a million took 10 us longer. One graph launch builds the batch at batchletIndex
 // with no host round trip and no conditional node; a stopped batch (memory,
 // no batch uploaded, time budget) runs through as no-ops.
 cudaError_t captureBatchGraph(const Dev& d, int pointGrid, int fixedGrid, int restGrid, cudaGraphExec_t* out) {
@@ -2947,11 +2961,11 @@ cudaError_t captureBatchGraph(const Dev& d, int pointGrid, int fixedGrid, int re
         if ((e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) break;
         capturing = true;
         k_batch_begin<<<1, 1, 0, cs>>>(d, 1u);
-        k_count_first<<<pointGrid, 256, 0, cs>>>(d, nullptr, 0u);
-        k_deep_book<<<1, 1024, 0, cs>>>(d);
-        k_deep_bin<<<pointGrid, 256, 0, cs>>>(d, nullptr, 0u);
-        k_deep_split<<<1, 1024, 0, cs>>>(d);
-        k_deep_move<<<pointGrid, 256, 0, cs>>>(d, nullptr, 0u);
+        if ((e = launchBehind(k_count_first, pointGrid, 256, 0, cs, d, nullptr, 0u)) != cudaSuccess) break;
+        if ((e = launchBehind(k_deep_book, 1, 1024, 0, cs, d)) != cudaSuccess) break;
+        if ((e = launchBehind(k_deep_bin, pointGrid, 256, 0, cs, d, nullptr, 0u)) != cudaSuccess) break;
+        if ((e = launchBehind(k_deep_split, 1, 1024, 0, cs, d)) != cudaSuccess) break;
+        if ((e = launchBehind(k_deep_move, pointGrid, 256, 0, cs, d, nullptr, 0u)) != cudaSuccess) break;
         if ((e = launchExpandRest(d, restGrid, cs)) != cudaSuccess) break;
         if ((e = cudaEventRecord(fork, cs)) != cudaSuccess) break;
         if ((e = cudaStreamWaitEvent(cs2, fork, 0)) != cudaSuccess) break;
@@ -2967,8 +2981,8 @@ cudaError_t captureBatchGraph(const Dev& d, int pointGrid, int fixedGrid, int re
         if ((e = cudaStreamWaitEvent(cs, joinLevels, 0)) != cudaSuccess) break;
         k_vox_lift<<<pointGrid, kLiftThreads, 0, cs>>>(d);
         k_vox_commit<<<fixedGrid, 256, 0, cs>>>(d);
-        k_alloc_voxels<<<fixedGrid, 256, 0, cs>>>(d);
-        k_vox_store<<<fixedGrid, 256, 0, cs>>>(d);
+        if ((e = launchBehind(k_alloc_voxels, fixedGrid, 256, 0, cs, d)) != cudaSuccess) break;
+        if ((e = launchBehind(k_vox_store, fixedGrid, 256, 0, cs, d)) != cudaSuccess) break;
         if ((e = cudaStreamWaitEvent(cs, join, 0)) != cudaSuccess) break;
         k_batch_end<<<1, 1, 0, cs>>>(d, kNone);
         if ((e = cudaGetLastError()) != cudaSuccess) break;
