@@ -1,5 +1,6 @@
-// Rasterize stage: frustum test, pixel-budget LOD cut, one block per visible
-// node, 64-bit depth|colour atomicMin splatting into a headless framebuffer.
+// Rasterize stage: frustum test, pixel-budget LOD cut, the visible nodes' samples
+// split over warps, 64-bit depth|colour atomicMin splatting into a headless
+// framebuffer.
 //
 // Restates kernels/remolod/remolod_render.cu:30-198 and
 // kernels/shared/remo_{math,framebuffer,draw}.cuh. The framebuffer packs

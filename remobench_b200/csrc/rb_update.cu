@@ -9,7 +9,8 @@
 // Parity-critical float arithmetic (quantisation, voxel centres) uses the
 // explicitly rounded intrinsics (__fsub_rn, __fmul_rn, __fdiv_rn, __fmaf_rn),
 // so nvcc cannot contract or approximate it; the CPU oracle performs the same
-// operations in the same order.
+// operations in the same order (its division is quotient() here, which rounds
+// as the division does).
 #include <cuda_runtime.h>
 
 #include <cstring>
@@ -2942,9 +2943,9 @@ void launchResetRoot(const Dev& d, int grid, cudaStream_t s) { k_reset_root<<<gr
 // itself is launched behind that one (launchBehind): a batch of 250,000 points
 // 101 -> 97 us, of a million 168 -> 165. Behind k_expand_rest, or before the
 // join of the levels branch, it gave nothing more; with that branch on the main
-// stream the batches of a million took 10 us longer. One graph launch builds the batch at batchletIndex
-// with no host round trip and no conditional node; a stopped batch (memory,
-// no batch uploaded, time budget) runs through as no-ops.
+// stream the batches of a million took 10 us longer. One graph launch builds the
+// batch at batchletIndex with no host round trip and no conditional node; a
+// stopped batch (memory, no batch uploaded, time budget) runs through as no-ops.
 cudaError_t captureBatchGraph(const Dev& d, int pointGrid, int fixedGrid, int restGrid, cudaGraphExec_t* out) {
     *out = nullptr;
     cudaStream_t cs = nullptr, cs2 = nullptr, cs3 = nullptr;
