@@ -643,7 +643,7 @@ rb_status rb_allocate(rb_ctx* c, const rb_cloud_meta* meta, uint64_t budget) {
     {
         rb::RefineScratch& r = c->refine;
         r.capacity = cfg.refine_voxel_capacity ? cfg.refine_voxel_capacity : 2097152u;
-        r.hashMask = std::max<uint32_t>(nextPow2(2ull * r.capacity), 8u) - 1u;
+        r.hashMask = nextPow2(2ull * r.capacity) - 1u;
         ALLOC(r.refSlot, N, "refinement node marks");
         ALLOC(r.voxNode, (uint64_t)N + 1, "refinement nodes");
         ALLOC(r.voxBase, (uint64_t)N + 1, "refinement voxel offsets");

@@ -41,7 +41,7 @@ __device__ __forceinline__ uint32_t cellOf(uint32_t x28, uint32_t y28, uint32_t 
 // The table's home slot of a (node slot << 21 | cell) key: 2 x 2 x 2 cells share
 // a 128-byte line (eight 16-byte slots), hashed together, the place within the
 // line mixed with the hash so that flat surfaces fill all eight; probing goes
-// from line to line at the same place.
+// from line to line at the same place (nextSlot).
 __device__ __forceinline__ uint32_t slotOf(unsigned long long key, uint32_t mask) {
     const uint32_t cell = (uint32_t)key & 0x1FFFFFu;
     const uint32_t place = (cell & 1u) | ((cell >> 6) & 2u) | ((cell >> 12) & 4u);
@@ -50,7 +50,6 @@ __device__ __forceinline__ uint32_t slotOf(unsigned long long key, uint32_t mask
     h *= 0xBF58476D1CE4E5B9ull;
     return (((uint32_t)(h >> 32) & ~7u) | (((uint32_t)(h >> 24) ^ place) & 7u)) & mask;
 }
-__device__ __forceinline__ uint32_t nextSlot(uint32_t slot, uint32_t mask) { return (slot + 8u) & mask; }
 
 // The cell a voxel of node `node` stands for, from its centre
 // nodeMin + size (c + 0.5) / 128 (half a cell from either boundary).
@@ -154,7 +153,7 @@ __global__ void __launch_bounds__(256) k_cf_index(Dev d, RefineScratch r) {
         r.entrySlot[e] = kNone;
         if (phys == kNone) continue;
         uint32_t slot = slotOf(key, r.hashMask);
-        for (uint32_t probe = 0; probe <= r.hashMask >> 3; probe++) {
+        for (uint32_t probe = 0; probe <= r.hashMask; probe++) {
             const unsigned long long prev = atomicCAS(&r.hash[slot].x, ~0ull, key);
             if (prev == ~0ull) {
                 r.hash[slot].y = e;
@@ -169,7 +168,7 @@ __global__ void __launch_bounds__(256) k_cf_index(Dev d, RefineScratch r) {
 
 __device__ __forceinline__ uint32_t findEntry(const RefineScratch& r, unsigned long long key) {
     uint32_t slot = slotOf(key, r.hashMask);
-    for (uint32_t probe = 0; probe <= r.hashMask >> 3; probe++) {
+    for (uint32_t probe = 0; probe <= r.hashMask; probe++) {
         const ulonglong2 kv = __ldg(&r.hash[slot]);
         if (kv.x == key) return (uint32_t)kv.y;
         if (kv.x == ~0ull) return kNone;

@@ -356,6 +356,13 @@ __device__ __forceinline__ uint32_t chunkOf(const Dev& d, uint32_t slot, uint32_
     }
     return q;
 }
+// The slot probed after `slot` in a cell table of mask + 1 slots (a power of two):
+// the same place of the next line of eight, after the last line the next place
+// of the first. From anywhere it comes through every slot before one again, so a
+// free slot is found wherever it is, in a table of one line or less too.
+__device__ __forceinline__ uint32_t nextSlot(uint32_t slot, uint32_t mask) {
+    return slot + 8u <= mask ? slot + 8u : (slot + 1u) & 7u & mask;
+}
 // Bump allocation of `units` 16-byte units; kNone when the arena is full.
 __device__ __forceinline__ uint32_t arenaAlloc(const Dev& d, uint32_t units) {
     const uint32_t off = atomicAdd(&d.ctr->arenaBump, units);
