@@ -1639,7 +1639,7 @@ __global__ void __launch_bounds__(1024, 1) k_expand_rest(Dev d) {
 // neighbouring points and a new cell's siblings meet in few lines; the place
 // within the line is mixed with the brick's hash so that flat surfaces, which
 // fill half of a brick, still spread over all eight. Probing goes from line to
-// line at the same place (nextLine), so a place's chain is as long as in a table
+// line at the same place (nextSlot), so a place's chain is as long as in a table
 // of an eighth of the size at the same load.
 __device__ __forceinline__ uint32_t hashSlot(unsigned long long key, uint32_t mask) {
     const uint32_t cell = (uint32_t)key & 0x1FFFFFu;
@@ -1650,7 +1650,6 @@ __device__ __forceinline__ uint32_t hashSlot(unsigned long long key, uint32_t ma
     h ^= h >> 32;
     return (((uint32_t)h & ~7u) | (((uint32_t)h ^ place) & 7u)) & mask;
 }
-__device__ __forceinline__ uint32_t nextLine(uint32_t slot, uint32_t mask) { return (slot + 8u) & mask; }
 
 // Records a claimed table slot in the batch's list of new cells.
 __device__ __forceinline__ void listNewCell(const Dev& d, uint32_t e, uint32_t slot) {
@@ -1685,7 +1684,7 @@ __device__ void hashInsertFrom(const Dev& d, unsigned long long key, unsigned lo
             else atomicCAS(vs, kHashEmpty, val);
             return;
         }
-        slot = nextLine(slot, d.hashMask);
+        slot = nextSlot(slot, d.hashMask);
     }
     atomicOr(&d.ctr->overflowFlags, (uint32_t)kOvfBacklog);
     d.ctr->hashNeedsClear = 1u;
@@ -1833,9 +1832,9 @@ __global__ void __launch_bounds__(256) k_vox_sample(Dev d, const Point* __restri
                 cur = atomicCAS(&d.hashSlots[slot].x, kHashEmpty, key);
                 claimed = cur == kHashEmpty;
                 update = claimed || cur == key;
-                if (!update) hashInsertFrom(d, key, val, nextLine(slot, d.hashMask));
+                if (!update) hashInsertFrom(d, key, val, nextSlot(slot, d.hashMask));
             } else {
-                hashInsertFrom(d, key, val, nextLine(slot, d.hashMask));
+                hashInsertFrom(d, key, val, nextSlot(slot, d.hashMask));
             }
             if (update) {
                 if (lowest) atomicMin(&d.hashSlots[slot].y, val);
@@ -1896,7 +1895,7 @@ __device__ __forceinline__ bool liftInsert(const Dev& d, unsigned long long key,
                 return atomicCAS(&d.hashSlots[slot].y, kHashEmpty, val) == kHashEmpty;
             }
         }
-        slot = nextLine(slot, d.hashMask);
+        slot = nextSlot(slot, d.hashMask);
     }
     atomicOr(&d.ctr->overflowFlags, (uint32_t)kOvfBacklog);
     d.ctr->hashNeedsClear = 1u;
@@ -2149,7 +2148,7 @@ __global__ void __launch_bounds__(256) k_vox_sample_levels(Dev d, const Point* _
                     if (lowest) atomicMin(&d.hashSlots[slot[j]].y, val);
                     else atomicCAS(&d.hashSlots[slot[j]].y, kHashEmpty, val);
                 } else if (state[j] == 3u) {
-                    hashInsertFrom(d, key[j], val, nextLine(slot[j], d.hashMask));
+                    hashInsertFrom(d, key[j], val, nextSlot(slot[j], d.hashMask));
                 }
             }
             // the claimed slots wait in the warp's buffer; 32 or more go to the
