@@ -487,13 +487,13 @@ __global__ void __launch_bounds__(256) k_wireframe(Dev d, Frame f, unsigned long
 // one wave of blocks, and remembers the pixels it has met; what is left is the
 // latency of the point loads, hence many warps (32 registers) with two points
 // each in flight: 47 us, against 77 with four points at four blocks per SM.
-template <bool kOnePixel>
+template <bool kOnePixel, bool kSeen>
 __global__ void __launch_bounds__(256, 8) k_raster_flat(Frame f, unsigned long long* fb,
                                                      const Point* __restrict__ pts, uint64_t n) {
     constexpr uint32_t kDraw = 2;
     __shared__ SeenPixels s_seen;
-    // a pixel index past 2^32 - 1 is left out of the table; ~0 marks no pixel
-    for (uint32_t i = threadIdx.x; i < (1u << kSeenBits); i += blockDim.x) s_seen.e[i] = ~0ull;
+    if (kSeen)  // ~0 marks no pixel: no depth is above its own
+        for (uint32_t i = threadIdx.x; i < (1u << kSeenBits); i += blockDim.x) s_seen.e[i] = ~0ull;
     __syncthreads();
     const uint64_t share = (n / gridDim.x + 32u) & ~31ull;
     const uint64_t begin = blockIdx.x * share, end = begin + share < n ? begin + share : n;
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(256, 8) k_raster_flat(Frame f, unsigned long l
             ok[j] = i < end;
             v[j] = ok[j] ? __ldg(reinterpret_cast<const float4*>(pts + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        drawPoints<kOnePixel, kOnePixel, kDraw>(fb, f, v, ok, true, 0u, s_seen.e);
+        drawPoints<kOnePixel, kSeen, kDraw>(fb, f, v, ok, true, 0u, s_seen.e);
     }
 }
 
@@ -625,8 +625,12 @@ void launchRaster(const Dev& d, const Frame& f, unsigned long long* fb, const Re
 }
 void launchRasterFlat(const Frame& f, unsigned long long* fb, const Point* pts, uint64_t n, int grid,
                       cudaStream_t s) {
-    if (f.pointSize / 2 == 0) k_raster_flat<true><<<grid, 256, 0, s>>>(f, fb, pts, n);
-    else k_raster_flat<false><<<grid, 256, 0, s>>>(f, fb, pts, n);
+    // the table of seen pixels names a pixel by 32 bits of its index: one-pixel
+    // splats in larger frames go without it
+    const bool indexed = (uint64_t)f.width * (uint64_t)f.height <= 1ull << 32;
+    if (f.pointSize / 2 != 0) k_raster_flat<false, false><<<grid, 256, 0, s>>>(f, fb, pts, n);
+    else if (indexed) k_raster_flat<true, true><<<grid, 256, 0, s>>>(f, fb, pts, n);
+    else k_raster_flat<true, false><<<grid, 256, 0, s>>>(f, fb, pts, n);
 }
 void launchEdl(unsigned long long* fb, uint32_t* rgba, uint32_t w, uint32_t h, float strength, cudaStream_t s) {
     // 32-row tiles while they are many waves of blocks, else 16-row ones: at

@@ -98,3 +98,38 @@ def test_flat_frame(c1_cloud, n, ps):
     ctx.render_flat(f, torch.from_numpy(cloud.view(np.float32).reshape(-1, 4)).cuda(), fb)
     assert np.array_equal(_u64(fb), ob.render_flat(cloud, oracle_frame(f)))
     ctx.close()
+
+
+def test_flat_frame_of_more_than_2_32_pixels():
+    """Points of one column in rows 32768 apart, 2^32 pixels in index: the nearer
+    ones hide nothing of the further ones. 34 GB of framebuffer."""
+    import torch
+    from remobench_b200 import capi
+    from remobench_b200.lod import Context
+    w, h, group, far_row = 131_072, 32_769, 1024, 32_768
+    f = capi.Frame()
+    f.width, f.height, f.lod_pixel_budget, f.point_size = float(w), float(h), 128.0, 1
+    for t in (f.transform, f.transform_frozen):
+        t[0] = t[5] = t[10] = t[14] = 1.0  # clip = (x, y, z, z)
+    for a in range(3):
+        f.box_min[a], f.box_max[a] = -4.0, 4.0
+    # 1,024 columns, each 512 points near in the first row, then 512 further in the last
+    i = np.arange(group * group)
+    col, far = (i // group) * 128, i % group >= group // 2
+    z = np.where(far, 2.0, 1.0)
+    p = np.zeros(len(i), dtype=ob.POINT_DTYPE)
+    p["x"] = ((2 * col + 1) / w - 1.0) * z
+    p["y"] = ((2 * np.where(far, far_row, 0) + 1) / h - 1.0) * z
+    p["z"] = z
+    p["color"] = np.where(far, 7, 3)
+    fb = torch.empty(w * h, dtype=torch.int64, device="cuda")
+    ctx = Context(pipeline=2)
+    ctx.allocate(len(p), (-4, -4, -4), (4, 4, 4))
+    ctx.render_flat(f, torch.from_numpy(p.view(np.float32).reshape(-1, 4)).cuda(), fb)
+    at = torch.arange(group, device="cuda") * 128
+    depth = {1.0: 0x3F800000, 2.0: 0x40000000}
+    assert np.all(_u64(fb[at]) == (depth[1.0] << 32 | 3))
+    assert np.all(_u64(fb[far_row * w + at]) == (depth[2.0] << 32 | 7))
+    ctx.close()
+    del fb, at
+    torch.cuda.empty_cache()
