@@ -154,6 +154,7 @@ __global__ void __launch_bounds__(kRollThreads) k_roll(Dev d, RollSum* roll, uin
                 const uint32_t inner = __popc(__ballot_sync(gmask, !leaf));
                 if (arrived != inner + 1u) break;
                 if (oct == 0u) rollArrive[g] = 0u;
+                __syncwarp(gmask);  // lane 0's acquire, for the others' reads
                 const unsigned long long* p = reinterpret_cast<const unsigned long long*>(&roll[node]);
 #pragma unroll
                 for (uint32_t k = 0; k < kRollWords; k++) words[oct][k] = __ldcg(p + k);
