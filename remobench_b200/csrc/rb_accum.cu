@@ -221,7 +221,8 @@ __device__ __forceinline__ void add128pair(unsigned long long& lo, unsigned long
 // than the two that 93 registers allow. Bound by instruction issue: 20M points
 // took 108 us with a division per coordinate, 64-bit clamps and a Morton
 // comparison per point, 77 us without (4.2 TB/s of the points read).
-__global__ void __launch_bounds__(kAccumThreads, 3) k_accumulate(Dev d, uint32_t batchIndex, int useList) {
+__global__ void __launch_bounds__(kAccumThreads, 3) k_accumulate(Dev d, uint32_t batchIndex, bool atCursor,
+                                                                int useList) {
     follow();
     __shared__ unsigned long long s_morton;
     const Counters* c = d.ctr;
@@ -229,7 +230,7 @@ __global__ void __launch_bounds__(kAccumThreads, 3) k_accumulate(Dev d, uint32_t
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t ppc = d.ppc, parts = c->accumParts, step = itemStep(d, parts);
     const unsigned long long bound = c->mortonBound;
-    if (batchIndex == kAtCursor) batchIndex = c->batchletIndex;
+    if (atCursor) batchIndex = c->batchletIndex;
     if (threadIdx.x == 0) s_morton = 0ull;
     __syncthreads();
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
@@ -410,10 +411,10 @@ __global__ void __launch_bounds__(256) k_accum_verify(Dev d) {
     }
 }
 
-void launchAccumulate(const Dev& d, uint32_t batchIndex, int useList, int grid, cudaStream_t s) {
+void launchAccumulate(const Dev& d, uint32_t batchIndex, bool atCursor, int useList, int grid, cudaStream_t s) {
     k_accum_begin<<<1, 1, 0, s>>>(d);
     launchBehind(k_accum_plan, grid / 4 + 1, 256, 0, s, d, useList);
-    launchBehind(k_accumulate, grid, kAccumThreads, 0, s, d, batchIndex, useList);
+    launchBehind(k_accumulate, grid, kAccumThreads, 0, s, d, batchIndex, atCursor, useList);
 }
 void launchAccumVerify(const Dev& d, int grid, cudaStream_t s) { launchBehind(k_accum_verify, grid, 256, 0, s, d); }
 

@@ -333,10 +333,10 @@ rb_status checkSync(rb_ctx* c) {
     return RB_OK;
 }
 
-// batchIndex rb::kAtCursor: the batches consumed so far, read on the device.
-rb_status accumulate(rb_ctx* c, uint32_t batchIndex) {
+// atCursor: the batches consumed so far, read on the device, instead of batchIndex.
+rb_status accumulate(rb_ctx* c, uint32_t batchIndex, bool atCursor = false) {
     const Dev& d = c->d;
-    LAUNCH(c, K_ACCUMULATE, 0, rb::launchAccumulate(d, batchIndex, c->accumAll ? 0 : 1, c->numSMs * 8, c->stream));
+    LAUNCH(c, K_ACCUMULATE, 0, rb::launchAccumulate(d, batchIndex, atCursor, c->accumAll ? 0 : 1, c->numSMs * 8, c->stream));
     LAUNCH(c, K_ACCUM_VERIFY, 0, rb::launchAccumVerify(d, c->numSMs * 2, c->stream));
     RB_CUDA(c, cudaGetLastError());
     c->accumAll = false;
@@ -733,7 +733,7 @@ static rb_status buildFrom(rb_ctx* c, const rb::Point* ring, const uint32_t* siz
         const uint64_t pointsBefore = c->hostCtr->numPointsProcessed;
         for (uint32_t k = 0; k < nb; k++) RB_CUDA(c, cudaGraphLaunch(c->batchGraph, c->stream));
         rb_status st = RB_OK;
-        if (accumOn && (st = accumulate(c, rb::kAtCursor)) != RB_OK) return st;
+        if (accumOn && (st = accumulate(c, 0, true)) != RB_OK) return st;
         RB_CUDA(c, cudaEventRecord(c->evStop, c->stream));
         if ((st = readCounters(c)) != RB_OK) return st;
         if ((st = checkSync(c)) != RB_OK) return st;

@@ -84,9 +84,8 @@ void launchSweep(const Dev& d, int grid, cudaStream_t s);
 void launchResetRoot(const Dev& d, int grid, cudaStream_t s);
 
 // Accumulate
-// batchIndex kAtCursor: Counters::batchletIndex.
-constexpr uint32_t kAtCursor = 0xFFFFFFFFu;
-void launchAccumulate(const Dev& d, uint32_t batchIndex, int useList, int grid, cudaStream_t s);
+// atCursor: Counters::batchletIndex takes batchIndex's place.
+void launchAccumulate(const Dev& d, uint32_t batchIndex, bool atCursor, int useList, int grid, cudaStream_t s);
 void launchAccumVerify(const Dev& d, int grid, cudaStream_t s);
 
 // Rasterize

@@ -60,3 +60,14 @@ def test_boxes(c1_cloud, shrink, scale):
         cloud[a] *= np.float32(scale)
     bmax = (np.asarray(bmax) * np.float32(scale) * np.float32(shrink)).astype(np.float32)
     _check(cloud, bmin, bmax, 20_011, max_points_per_node=2000, store_capacity=4 << 30)
+
+
+def test_any_batch_index(c1_cloud):
+    """What a caller gives as the batch index is what the touched leaves record."""
+    _, cloud, bmin, bmax = c1_cloud
+    ctx, _ = build_gpu(np.ascontiguousarray(cloud[:9_001]), bmin, bmax, 9_001, accumulate=0)
+    ctx.accumulate(0xFFFFFFFF)
+    sums = ctx.accums()
+    assert int(sums["count"].sum()) == 9_001
+    assert np.all(sums["last_touched_batch"][sums["count"] > 0] == 0xFFFFFFFF)
+    ctx.close()
