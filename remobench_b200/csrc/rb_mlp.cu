@@ -64,9 +64,12 @@ __device__ __forceinline__ float gelu(float z) {
 // below the tanhf form's (9.3e-9 against 1.8e-8 on [-3, 0), 4.5e-8 against
 // 5.9e-8 on [0, 3); derivative 1.6e-8 against 3.7e-8, 5.7e-8 against 5.2e-8,
 // and 4.5e-8 against 1.9e-7 on [3, 6)), at half the instructions: the two GELUs
-// were most of the gradient kernel's.
+// were most of the gradient kernel's. +infinity (a sum past FP32's range) is taken
+// as the largest float, which the caller's rounding to BF16 makes +infinity again,
+// as the tanhf form gives; |z| r would be infinity times zero. A NaN stays one.
 __device__ __forceinline__ float geluGrad(float z, float& dgelu) {
     const float c = 0.7978845608028654f;
+    asm("min.NaN.f32 %0, %0, 0f7F7FFFFF;" : "+f"(z));
     const float zz = z * z;
     const float u = c * (z + 0.044715f * zz * z);
     const float p = expf(-2.0f * fabsf(u));

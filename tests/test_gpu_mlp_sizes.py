@@ -47,3 +47,20 @@ def test_steps_and_gradients_do_not_mix():
         assert np.max(np.abs(a.mlp_params() - b.mlp_params())) <= 2e-3 * 3e-3 * (step + 1) + 1e-6
     a.close()
     b.close()
+
+
+def test_loss_of_an_overflowed_activation():
+    """Hidden sums past FP32's range are +infinity, and so is their GELU: the loss
+    is infinite, not undefined."""
+    import torch
+    from mlp_reference import OFF
+    ctx = _context(1)
+    p = np.zeros(len(ctx.mlp_params()), dtype=np.float32)
+    for k in ("W1", "W2"):
+        p[OFF[k]:OFF["b" + k[1]]] = 1.0
+    p[OFF["W3"]:OFF["W3"] + 64], p[OFF["W3"] + 64:OFF["b3"]] = 1.0, -1.0
+    ctx.mlp_set_params(p)
+    x = torch.full((3, 16), 3.0e38, device="cuda")
+    t = torch.tensor([[0.0, 1.0]], device="cuda").repeat(3, 1)
+    assert ctx.mlp_gradients(x, t)[1] == float("inf")
+    ctx.close()
