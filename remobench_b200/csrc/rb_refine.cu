@@ -188,6 +188,7 @@ __device__ __forceinline__ uint32_t unitPoints(uint32_t ppc) { return ppc >= kCf
 // Dev::accumItem the leaf's first unit (Accumulate's plan, free between folds).
 __global__ void __launch_bounds__(256) k_cf_units(Dev d, RefineScratch r) {
     const uint32_t nn = d.ctr->numNodes, unit = unitPoints(d.ppc);
+    const bool arenaFull = (d.ctr->overflowFlags & (uint32_t)kOvfArena) != 0u;
     unsigned long long visited = 0;
     for (uint32_t leaf = blockIdx.x * blockDim.x + threadIdx.x; leaf < nn; leaf += gridDim.x * blockDim.x) {
         const uint32_t np = min(d.numPoints[leaf], d.numPointChunks[leaf] * d.ppc);
@@ -203,7 +204,13 @@ __global__ void __launch_bounds__(256) k_cf_units(Dev d, RefineScratch r) {
             m++;
             withVoxels |= r.voxBase[k + 1u] - r.voxBase[k];
         }
-        visited += (unsigned long long)np * m;
+        uint32_t held = np;
+        if (arenaFull && m > 0u) {  // points whose chunk the arena had no room for are not there
+            const uint32_t off = d.ptTableOff[leaf];
+            for (uint32_t k = 0; k <= (np - 1u) / d.ppc; k++)
+                if (d.tablePool[off + k] == kNone) held -= min(d.ppc, np - k * d.ppc);
+        }
+        visited += (unsigned long long)held * m;
         if (withVoxels == 0u) continue;
         const uint32_t units = (np + unit - 1u) / unit, first = atomicAdd(&r.ctr->units, units);
         d.accumItem[leaf] = first;

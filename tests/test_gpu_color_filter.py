@@ -42,3 +42,20 @@ def test_filtered_colours_equal_the_oracle(c1_cloud, points, ppc, limit, shrink,
         assert r.points_visited == int((above * nodes["num_points"])[nodes["is_leaf"] == 1].sum())
     ctx.close()
     tree.close()
+
+
+def test_points_visited_where_chunks_are_missing(c1_cloud):
+    """A batch larger than the arena: the points without a chunk are dropped and
+    not counted as visited."""
+    from remobench_b200.lod import make_frame
+    _, cloud, bmin, bmax = c1_cloud
+    cloud = np.ascontiguousarray(np.concatenate([cloud, cloud[:900_000]]))
+    ctx, _ = build_gpu(cloud, bmin, bmax, len(cloud), store_capacity=1 << 20, safety_margin=0)
+    s = ctx.stats()
+    assert s.overflow_flags & 8 and 0 < s.dropped_points < len(cloud)
+    f = make_frame(bmin, bmax, 1920, 1080, yaw=1.3, pitch=-0.5, radius_scale=0.5)
+    ctx.analyze(f, min_points=int(0.6 * len(cloud)), frontier_only=False)
+    assert ctx.queue().tolist() == [0]
+    r = ctx.refine_colors(1)
+    assert r.nodes_filtered == 1 and r.points_visited == len(cloud) - s.dropped_points
+    ctx.close()
