@@ -33,12 +33,31 @@ struct RenderScratch {
 constexpr uint32_t kDrawCountBits = 24;
 constexpr unsigned long long kDrawCountMask = (1ull << kDrawCountBits) - 1ull;
 
-// A draw list entry: the node, and the stored samples of the items before it (a
-// sample takes an arena unit, and there are fewer than 2^32).
+// A draw list entry: the node in the low kDrawNodeBits bits (ids are below 2^21),
+// the stored samples of the items before it above them. Together they can pass
+// 2^32: past an arena overflow points without a chunk count too.
 struct DrawItem {
-    uint32_t node;
-    uint32_t first;
+    unsigned long long bits;
 };
+constexpr uint32_t kDrawNodeBits = 21;
+__host__ __device__ inline DrawItem drawItem(uint32_t node, unsigned long long first) {
+    return DrawItem{first << kDrawNodeBits | node};
+}
+__host__ __device__ inline uint32_t itemNode(DrawItem it) { return (uint32_t)it.bits & ((1u << kDrawNodeBits) - 1u); }
+__host__ __device__ inline unsigned long long itemFirst(DrawItem it) { return it.bits >> kDrawNodeBits; }
+
+// The samples [begin, end) of a frame's `total` that warp w of `warps` draws.
+struct DrawShare {
+    unsigned long long begin, end;
+};
+__host__ __device__ inline DrawShare drawShare(unsigned long long total, uint32_t warps, uint32_t w) {
+    const unsigned long long share = ((total + warps - 1u) / warps + 31ull) & ~31ull, begin = w * share;
+    return begin >= total ? DrawShare{total, total} : DrawShare{begin, total - begin < share ? total : begin + share};
+}
+// The first sample of an item of n that a share ending at `end` leaves.
+__host__ __device__ inline uint32_t itemStop(DrawItem it, uint32_t n, unsigned long long end) {
+    return end - itemFirst(it) < n ? (uint32_t)(end - itemFirst(it)) : n;
+}
 
 // What a render reports, in pinned host memory that k_raster writes.
 struct RenderResult {

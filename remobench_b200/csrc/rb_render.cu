@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(256) k_cut(Dev d, Frame f, unsigned long long*
         at = __shfl_sync(0xFFFFFFFFu, at, 31);
         const uint32_t idx = (uint32_t)(at & kDrawCountMask) + (uint32_t)__popc(em & ((1u << lane) - 1u));
         const bool listed = emit && idx < cap;
-        if (listed) items[idx] = DrawItem{i, (uint32_t)((at >> kDrawCountBits) + pre - work)};
+        if (listed) items[idx] = drawItem(i, (at >> kDrawCountBits) + pre - work);
         unsigned long long drawn = listed ? (unsigned long long)np + nv : 0ull;
 #pragma unroll
         for (uint32_t o = 16; o > 0u; o >>= 1) drawn += __shfl_xor_sync(0xFFFFFFFFu, drawn, o);
@@ -347,33 +347,34 @@ __global__ void __launch_bounds__(256, 6) k_raster(Dev d, Frame f, unsigned long
         host->samples = rs->samples;
     }
     if (ni == 0u) return;
-    uint32_t total = (uint32_t)(rs->cursor >> kDrawCountBits);
-    if ((rs->cursor & kDrawCountMask) > cap)  // the list is full: its last item ends the work
-        total = items[ni - 1u].first + storedPoints(d, items[ni - 1u].node) + storedVoxels(d, items[ni - 1u].node);
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5, w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t share = (uint32_t)(((((unsigned long long)total + warps - 1u) / warps) + 31ull) & ~31ull);
-    const unsigned long long begin64 = (unsigned long long)w * share;
-    if (begin64 >= total) return;
-    const uint32_t begin = (uint32_t)begin64, end = total - begin < share ? total : begin + share;
+    unsigned long long total = rs->cursor >> kDrawCountBits;
+    if ((rs->cursor & kDrawCountMask) > cap) {  // the list is full: its last item ends the work
+        const DrawItem last = items[ni - 1u];
+        total = itemFirst(last) + storedPoints(d, itemNode(last)) + storedVoxels(d, itemNode(last));
+    }
+    const DrawShare mine =
+        drawShare(total, (gridDim.x * blockDim.x) >> 5, (blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (mine.begin >= mine.end) return;
+    const unsigned long long begin = mine.begin, end = mine.end;
     // the last item that starts at or before `begin`: [lo, hi) narrows 32-fold a round
     uint32_t lo = 0, hi = ni;
     while (hi - lo > 1u) {
         const uint32_t step = (hi - lo + 31u) >> 5;
         const uint32_t p = lo + lane * step;
-        const bool le = p < hi && items[p].first <= begin;
+        const bool le = p < hi && itemFirst(items[p]) <= begin;
         const uint32_t k = 31u - (uint32_t)__clz((int)__ballot_sync(0xFFFFFFFFu, le));
         lo += k * step;
         hi = min(hi, lo + step);
     }
     const bool rgb = f.colorMode < 1 || f.colorMode > 3;
-    for (uint32_t s = begin; s < end; lo++) {
+    for (unsigned long long s = begin; s < end; lo++) {
         const DrawItem it = items[lo];
-        const uint32_t node = it.node;
+        const uint32_t node = itemNode(it);
         const uint32_t np = storedPoints(d, node), n = np + storedVoxels(d, node);
         const uint32_t poff = d.ptTableOff[node], voff = d.vxTableOff[node];
         const uint32_t fixed = rgb ? 0u : itemColor(f.colorMode, node, d.level[node]);
-        const uint32_t stop = min(n, end - it.first);
-        for (uint32_t k0 = s - it.first; k0 < stop; k0 += 32u * kDraw) {
+        const uint32_t stop = itemStop(it, n, end);
+        for (uint32_t k0 = (uint32_t)(s - itemFirst(it)); k0 < stop; k0 += 32u * kDraw) {
             float4 v[kDraw];
             bool ok[kDraw];
 #pragma unroll
@@ -389,7 +390,7 @@ __global__ void __launch_bounds__(256, 6) k_raster(Dev d, Frame f, unsigned long
             }
             drawPoints<kOnePixel, false, kDraw>(fb, f, v, ok, rgb, fixed, nullptr);
         }
-        s = it.first + stop;
+        s = itemFirst(it) + stop;
     }
 }
 
@@ -463,7 +464,7 @@ __global__ void __launch_bounds__(256) k_wireframe(Dev d, Frame f, unsigned long
     const float cube = fmaxf(fmaxf(f.boxMax[0] - f.boxMin[0], f.boxMax[1] - f.boxMin[1]), f.boxMax[2] - f.boxMin[2]);
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < (uint64_t)ni * 12u;
          i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t node = items[i / 12u].node;
+        const uint32_t node = itemNode(items[i / 12u]);
         const uint32_t edge = (uint32_t)(i % 12u);
         const uint32_t lv = d.level[node];
         const float size = cube / __int_as_float((int)((127u + lv) << 23));
