@@ -78,11 +78,13 @@ __device__ __forceinline__ void atomicAdd128(unsigned long long* lo, unsigned lo
     if (vhi + carry) atomicAdd(hi, vhi + carry);
 }
 
-// The largest fold whose chunks are cut into kAccumParts items. A warp per whole
+// The largest fold whose items are cut into kAccumParts parts, a warp each. A warp per whole
 // chunk leaves most of the 3,552 resident warps without work below about this
 // many points (100,000 points: 18.2 us in whole chunks, 8.3 in quarters); above,
 // an item's reduction, about 20 points' worth, is better spent on a whole one.
 constexpr unsigned long long kAccumFine = 3000000ull;
+constexpr uint32_t kAccumParts = 4;
+static_assert(kAccumThreads / 32 % kAccumParts == 0, "a block's warps count the parts off");
 
 // Starts a fold: its counters to zero (RemolodPipeline.cpp:251-256 restarts the
 // globals per launch), and how its chunks are cut, from the points that came in
@@ -102,12 +104,6 @@ __global__ void k_accum_begin(Dev d) {
     c->mortonBound = 0;
 }
 
-// Slots per item, and the item a slot falls in: parts items per chunk.
-__device__ __forceinline__ uint32_t itemStep(const Dev& d, uint32_t parts) { return (d.ppc + parts - 1u) / parts; }
-__device__ __forceinline__ uint32_t itemOf(const Dev& d, uint32_t slot, uint32_t parts, uint32_t step) {
-    return slot / d.ppc * parts + slot % d.ppc / step;
-}
-
 __device__ __forceinline__ unsigned long long mortonCode(uint32_t x, uint32_t y, uint32_t z) {
     return (mortonSpread(x) << 2) | (mortonSpread(y) << 1) | mortonSpread(z);
 }
@@ -115,11 +111,12 @@ __device__ __forceinline__ unsigned long long mortonCode(uint32_t x, uint32_t y,
 // The fold's plan: the nodes to visit (the dirty list, or every node), each
 // leaf's new range [count, min(numPoints, capacity)) read before any fold
 // updates count, and each node's work items. An inner node with sums is one
-// item (cleared); a leaf with new points one item per point chunk, or part of
-// one (Counters::accumParts), its new range touches. Sums are exact, so the order of items is free: each block
-// claims a contiguous run of item indices with one atomic (Counters::
-// accumItems) and writes every item's plan entry,
-// so a warp of the fold finds its item with one load. Items can pass
+// item (cleared); a leaf with new points one item per point chunk its new range
+// touches. Sums are exact, so the order of items is free: each block claims a
+// contiguous run of item indices with one atomic (Counters::accumItems) and
+// writes every item's plan entry, so a warp of the fold finds its item with one
+// load. The parts of an item (Counters::accumParts) are not listed: the fold's
+// warps count them off, and a part without a new point is skipped. Items can pass
 // accumUnitCap (every live point chunk plus every node) only once the arena
 // has run out (RB_OVF_ARENA): those are not folded. Folded-leaf and point
 // totals are added per block. The watermark needs only the leaves that can hold
@@ -132,7 +129,6 @@ __global__ void __launch_bounds__(256) k_accum_plan(Dev d, int useList) {
     __shared__ uint32_t s_base, s_leaves;
     __shared__ unsigned long long s_points, s_bound;
     Counters* c = d.ctr;
-    const uint32_t parts = c->accumParts, step = itemStep(d, parts);
     const uint32_t total = useList ? (c->numDirty < d.maxNodes ? c->numDirty : d.maxNodes) : c->numNodes;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
@@ -155,7 +151,7 @@ __global__ void __launch_bounds__(256) k_accum_plan(Dev d, int useList) {
                 const uint32_t np = d.numPoints[node];
                 to = np < cap ? np : cap;
                 if (to > from) {
-                    items = itemOf(d, to - 1u, parts, step) - itemOf(d, from, parts, step) + 1u;
+                    items = (to - 1u) / d.ppc - from / d.ppc + 1u;
                     const uint32_t sh = (uint32_t)kMaxDepth - d.level[node];
                     atomicMax(&s_bound, mortonCode(d.nodeX[node] << sh, d.nodeY[node] << sh, d.nodeZ[node] << sh));
                     atomicAdd(&s_leaves, 1u);
@@ -228,30 +224,32 @@ __global__ void __launch_bounds__(kAccumThreads, 3) k_accumulate(Dev d, uint32_t
     const Counters* c = d.ctr;
     const uint32_t items = c->accumItems;
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t ppc = d.ppc, parts = c->accumParts, step = itemStep(d, parts);
+    const uint32_t ppc = d.ppc, parts = c->accumParts, step = (ppc + parts - 1u) / parts;
     const unsigned long long bound = c->mortonBound;
     if (atCursor) batchIndex = c->batchletIndex;
     if (threadIdx.x == 0) s_morton = 0ull;
     __syncthreads();
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    // a block's warps, and so the grid's, are a multiple of the parts
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t part = warp % parts;
     unsigned long long blockMax = 0ull;  // lane 0's running watermark
-    for (uint32_t it = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < items; it += warps) {
+    for (uint32_t it = warp / parts; it < items; it += warps / parts) {
         if (it >= d.accumUnitCap) break;  // only past an arena overflow (see k_accum_plan)
         const uint32_t w = d.accumUnitW[it];
         const uint32_t node = useList ? d.dirtyList[w] : w;
         AccumI* a = &d.accum[node];
         const uint32_t from0 = d.accumFrom[w], to = d.accumTo[w];
         if (to == from0) {  // an inner node holding sums
-            if (lane == 0) {
+            if (lane == 0 && part == 0u) {
                 AccumI z = {};
                 *a = z;
             }
             continue;
         }
-        const uint32_t part = itemOf(d, from0, parts, step) + (it - d.accumItem[w]);
-        const uint32_t ci = part / parts, lo = ci * ppc + part % parts * step;
+        const uint32_t ci = from0 / ppc + (it - d.accumItem[w]), lo = ci * ppc + part * step;
         const uint32_t from = max(from0, lo);
         const uint32_t end = min(to, min(lo + step, (ci + 1u) * ppc));
+        if (from >= end) continue;
         const uint32_t lv = d.level[node];
         const uint32_t sh = 28u - lv;
         const uint32_t lim = 1u << sh;

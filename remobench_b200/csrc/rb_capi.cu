@@ -608,7 +608,7 @@ rb_status rb_allocate(rb_ctx* c, const rb_cloud_meta* meta, uint64_t budget) {
     ALLOC(d.accumFrom, N, "accumulate plan ranges");
     ALLOC(d.accumTo, N, "accumulate plan ranges");
     ALLOC(d.accumItem, (uint64_t)N + 1, "accumulate plan items");
-    d.accumUnitCap = (uint32_t)std::min<uint64_t>((uint64_t)d.maxPtChunks * rb::kAccumParts + N, UINT32_MAX);
+    d.accumUnitCap = (uint32_t)std::min<uint64_t>((uint64_t)d.maxPtChunks + N, UINT32_MAX);
     ALLOC(d.accumUnitW, d.accumUnitCap, "accumulate work items");
     ALLOC(d.hist8, (uint64_t)N * 8, "child-octant counts");
     ALLOC(d.arrive, N, "points reaching each leaf");
@@ -647,8 +647,15 @@ rb_status rb_allocate(rb_ctx* c, const rb_cloud_meta* meta, uint64_t budget) {
         ALLOC(r.refSlot, N, "refinement node marks");
         ALLOC(r.voxNode, (uint64_t)N + 1, "refinement nodes");
         ALLOC(r.voxBase, (uint64_t)N + 1, "refinement voxel offsets");
-        ALLOC(r.acc, r.capacity, "refinement colour sums");
-        ALLOC(r.up, r.capacity, "refinement colour sums from below");
+        // the colour sums lie in the spill list, which holds nothing between
+        // batches, where it has the room (it does by default)
+        if ((uint64_t)d.spillCap * sizeof(rb::Point) >= 2ull * r.capacity * sizeof(ulonglong4)) {
+            r.acc = reinterpret_cast<ulonglong4*>(d.spillPts);
+            r.up = r.acc + r.capacity;
+        } else {
+            ALLOC(r.acc, r.capacity, "refinement colour sums");
+            ALLOC(r.up, r.capacity, "refinement colour sums from below");
+        }
         ALLOC(r.entrySlot, r.capacity, "refinement entry slots");
         ALLOC(r.upSlot, (uint64_t)N + 1, "refinement nodes' next filtered nodes");
         ALLOC(r.hash, (uint64_t)r.hashMask + 1, "refinement cell table");

@@ -90,7 +90,7 @@ struct Counters {
     uint32_t hashNeedsClear;      // the cell table holds entries its list cannot name
     uint32_t callBatches;         // batches built since the build call began
     uint32_t accumItems;          // work items of the current Accumulate launch
-    uint32_t accumParts;          // items a point chunk is cut into (k_accum_begin)
+    uint32_t accumParts;          // parts each of them is cut into (k_accum_begin)
     unsigned long long accumMark;   // points processed and spilled when the last Accumulate began
     unsigned long long mortonBound; // no new point's leaf with a Morton code above this is left out of the watermark
     uint32_t numZero;             // grids of nodes split this batch, to zero after expand
@@ -247,7 +247,7 @@ struct Dev {
     uint32_t* accumTo;       // [maxNodes]
     uint32_t* accumItem;     // [maxNodes + 1] exclusive prefix of work items
     uint32_t* accumUnitW;    // [accumUnitCap] plan entry of each work item
-    uint32_t accumUnitCap;   // kAccumParts per point chunk + nodes: every fold's items fit
+    uint32_t accumUnitCap;   // point chunks + nodes: every fold's items fit
     uint32_t* zeroList;      // [zeroCap] grids to zero after the expand loop
     // per node, its points per child octant, counted by the recount for the
     // nodes made by the last split: one level of lookahead for the next split
@@ -290,8 +290,6 @@ struct Dev {
     float octreeSize;
     float octreeRecip;       // 1 / octreeSize rounded to nearest, 0: divide (see quotient)
 };
-
-constexpr uint32_t kAccumParts = 4;  // items a chunk is cut into when a fold is small
 
 constexpr uint32_t kGridUnits = (uint32_t)(kGridBytes / 16u);
 

@@ -71,3 +71,14 @@ def test_any_batch_index(c1_cloud):
     assert int(sums["count"].sum()) == 9_001
     assert np.all(sums["last_touched_batch"][sums["count"] > 0] == 0xFFFFFFFF)
     ctx.close()
+
+
+@pytest.mark.parametrize("ppc,limit", [(1000, 1_743_378_284), (10, 1_853_000_612)])
+def test_memory_of_a_context(ppc, limit):
+    """What a context of the default sizes takes for 2M points with whole chunks as
+    work items and colour filtering's sums outside the spill list; no more now."""
+    from remobench_b200.lod import Context
+    ctx = Context(points_per_chunk=ppc)
+    ctx.allocate(2_000_000, (0, 0, 0), (1, 1, 1))
+    assert ctx.stats().bytes_allocated <= limit
+    ctx.close()

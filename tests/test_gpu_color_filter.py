@@ -5,7 +5,7 @@ that admits part of the queue."""
 import numpy as np
 import pytest
 
-from gpu_helpers import build_gpu, build_oracle, compare_voxels
+from gpu_helpers import build_gpu, build_oracle, compare_nodes, compare_voxels
 
 pytestmark = pytest.mark.gpu
 
@@ -59,3 +59,32 @@ def test_points_visited_where_chunks_are_missing(c1_cloud):
     r = ctx.refine_colors(1)
     assert r.nodes_filtered == 1 and r.points_visited == len(cloud) - s.dropped_points
     ctx.close()
+
+
+# 25,000 voxels' sums are exactly as long as the list of 100,000 spilled points
+@pytest.mark.parametrize("capacity", [25_000, 25_001])
+def test_sums_in_the_spill_list_and_beside_it(c1_cloud, capacity):
+    """Batches before, between and after filterings equal the oracle's."""
+    from remobench_b200.lod import DeviceRing, make_frame
+    _, cloud, bmin, bmax = c1_cloud
+    cloud = np.ascontiguousarray(cloud[::16])
+    cfg = dict(max_points_per_node=2000)
+    step = 30_000
+    ctx, _ = build_gpu(cloud[:step], bmin, bmax, step, spilled_capacity=100_000, refine_voxel_capacity=capacity, **cfg)
+    tree = build_oracle(cloud[:step], bmin, bmax, step, **cfg)
+    ring = DeviceRing(cloud, step, slots=ctx.cfg.ring_slots, slot_capacity=step)
+    ring.upload_window(0)
+    f = make_frame(bmin, bmax, 1920, 1080, yaw=1.3, pitch=-0.5, radius_scale=0.5)
+    for k in range(1, 4):
+        ctx.analyze(f, min_points=1, frontier_only=False)
+        queue = ctx.queue()
+        r = ctx.refine_colors(len(queue))
+        assert (r.nodes_filtered, r.voxels_filtered) == tree.refine_colors(queue, capacity=capacity)
+        assert r.voxels_filtered > 0
+        ctx.build(ring.ring, ring.sizes, k + 1, ring.num_batches)
+        tree.add_batch(cloud[k * step:(k + 1) * step])
+        tree.sweep()
+        nodes = compare_nodes(ctx, tree)
+        compare_voxels(ctx, tree, nodes)
+    ctx.close()
+    tree.close()
