@@ -134,3 +134,26 @@ def test_read_backs_follow_every_change(c1_cloud):
         assert r.batches_consumed == 4 and len(ctx.nodes()) == ctx.stats().num_nodes > 1
         assert int(ctx.accums()["count"].sum()) == len(cloud)
         ctx.close()
+
+
+def test_mask_after_more_candidates_than_the_sort_holds(c1_cloud):
+    """Then the queue keeps some of the candidates, and the mask marks those alone."""
+    import torch
+    _, cloud, bmin, bmax = c1_cloud
+    cloud = np.ascontiguousarray(cloud[:400_000])
+    ctx, _ = build_gpu(cloud, bmin, bmax, 100_000, max_points_per_node=30, store_capacity=6 << 30,
+                       backlog_capacity=4_000_000)
+    from remobench_b200.lod import make_frame
+    f = make_frame(bmin, bmax, 1920, 1080, yaw=1.2, pitch=-0.5, radius_scale=0.5)
+    r = ctx.analyze(f, min_points=1, frontier_only=False, queue_capacity=16_384)
+    q = ctx.queue()
+    assert r.overflow == 1 and len(q) == 16_384 and len(set(q.tolist())) == len(q)
+    mask = torch.full((ctx.cfg.max_nodes,), 7, dtype=torch.uint8, device="cuda")
+    for budget in (1, 5000, 16_384):
+        torch.cuda.synchronize()
+        ctx.refine(budget, mask)
+        m = mask.cpu().numpy()
+        nn = ctx.stats().num_nodes
+        assert set(np.nonzero(m[:nn])[0].tolist()) == set(q[:budget].tolist())
+        assert np.all(m[:nn] <= 1) and np.all(m[nn:] == 7)
+    ctx.close()
