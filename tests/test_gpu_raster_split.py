@@ -133,3 +133,23 @@ def test_flat_frame_of_more_than_2_32_pixels():
     ctx.close()
     del fb, at
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("ps", [-5, 0, 2, 4, 5, 7, 8, 10, 25, 1000])
+def test_splats_of_any_size(c1_cloud, ps):
+    """Rows of a splat around four pixels, wider than the frame, of no size."""
+    import torch
+    _, cloud, bmin, bmax = c1_cloud
+    cloud = np.ascontiguousarray(cloud[::4000])
+    ctx, _ = build_gpu(cloud, bmin, bmax, 200, max_points_per_node=50)
+    tree = build_oracle(cloud, bmin, bmax, 200, max_points_per_node=50)
+    pts = torch.from_numpy(cloud.view(np.float32).reshape(-1, 4)).cuda()
+    for w, h in ((1, 1), (61, 37), (320, 200)):
+        f = _frame(bmin, bmax, w, h, budget=40.0, point_size=ps)
+        fb, _ = _buffers(w, h)
+        ctx.render(f, fb)
+        assert np.array_equal(_u64(fb), tree.render(oracle_frame(f))[0])
+        ctx.render_flat(f, pts, fb)
+        assert np.array_equal(_u64(fb), ob.render_flat(cloud, oracle_frame(f)))
+    ctx.close()
+    tree.close()
