@@ -78,11 +78,14 @@ __device__ __forceinline__ void atomicAdd128(unsigned long long* lo, unsigned lo
     if (vhi + carry) atomicAdd(hi, vhi + carry);
 }
 
-// The largest fold whose items are cut into kAccumParts parts, a warp each. A warp per whole
-// chunk leaves most of the 3,552 resident warps without work below about this
-// many points (100,000 points: 18.2 us in whole chunks, 8.3 in quarters); above,
-// an item's reduction, about 20 points' worth, is better spent on a whole one.
-constexpr unsigned long long kAccumFine = 3000000ull;
+// The fold whose items, point chunks, are cut into kAccumParts parts, a warp each:
+// of fewer new points than kAccumFine whole chunks hold, and with at least a warp's
+// width of points a part. A warp per whole chunk leaves most of the 3,552 resident
+// warps without work below that (100,000 points in chunks of 1,000: 18.2 us whole,
+// 8.3 in quarters); above, and in small chunks, an item's reduction, about 20
+// points' worth, is better spent on a whole one (2M points in chunks of 7: 540 us
+// whole, 1,817 in quarters).
+constexpr uint32_t kAccumFine = 3000;
 constexpr uint32_t kAccumParts = 4;
 static_assert(kAccumThreads / 32 % kAccumParts == 0, "a block's warps count the parts off");
 
@@ -98,7 +101,8 @@ __global__ void k_accum_begin(Dev d) {
     g->numLeavesFolded = 0;
     g->innerWithSums = 0;
     const unsigned long long seen = c->numPointsProcessed + c->spilledPointsTotal;
-    c->accumParts = seen - c->accumMark < kAccumFine ? kAccumParts : 1u;
+    const bool fine = d.ppc >= 32u * kAccumParts && seen - c->accumMark < (unsigned long long)kAccumFine * d.ppc;
+    c->accumParts = fine ? kAccumParts : 1u;
     c->accumMark = seen;
     c->accumItems = 0;
     c->mortonBound = 0;

@@ -82,3 +82,17 @@ def test_memory_of_a_context(ppc, limit):
     ctx.allocate(2_000_000, (0, 0, 0), (1, 1, 1))
     assert ctx.stats().bytes_allocated <= limit
     ctx.close()
+
+
+# the smallest chunks that are cut are of 128 points, in folds of under 3,000 chunks
+@pytest.mark.parametrize("ppc,limit", [(5, 300), (127, 300), (128, 300), (129, 1000), (130, 50_000)])
+def test_items_around_the_smallest_cut_chunk(c1_cloud, ppc, limit):
+    _, cloud, bmin, bmax = c1_cloud
+    _check(np.ascontiguousarray(cloud[:80_003]), bmin, bmax, 9_001, points_per_chunk=ppc, max_points_per_node=limit,
+           store_capacity=4 << 30)
+
+
+def test_fold_above_the_fine_limit_of_small_chunks(c1_cloud):
+    _, cloud, bmin, bmax = c1_cloud
+    _check(np.ascontiguousarray(cloud), bmin, bmax, 300_001, points_per_chunk=128, max_points_per_node=5000,
+           store_capacity=8 << 30)
