@@ -9,10 +9,11 @@
 // found through a table keyed by (filtered node, cell):
 //   k_cf_plan   the queue prefix whose voxels fit the capacity, each node's
 //               first entry (one block);
-//   k_cf_index  every entry's cell from its voxel's centre into the table;
 //   k_cf_units  the leaves below a filtered node, cut into units of points;
+//   k_cf_index  every entry's cell from its voxel's centre into the table;
 //   k_cf_gather a unit's points summed per cell of the deepest filtered node
-//               above them, first in shared memory, then into its entries;
+//               above them, first in shared memory, then into its entries (or,
+//               with few points a voxel, every point into its entries: perPoint);
 //   k_cf_roll   every entry's sums into the entries of the filtered nodes above:
 //               a point's cell in an ancestor is a prefix of its cell below;
 //   k_cf_apply  means (rounded half up, alpha kept) written into the voxels,
@@ -120,12 +121,23 @@ __global__ void __launch_bounds__(1024) k_cf_plan(Dev d, RefineScratch r, const 
         r.ctr->nodes = m;
         r.ctr->voxels = total;
         r.ctr->points = 0;
+        r.ctr->pairs = 0;
         r.ctr->units = 0;
     }
 }
 
+// Whether the call adds each point to its entries one by one: with few points a
+// voxel, as in a cloud that fills its volume, most cells hold one, and summing them
+// per cell first, then upwards, is only more work. 2M points spread evenly, 1.6M
+// voxels, 1.2 points each: 358 us per cell, 275 per point; 1.3M voxels, 4.6 points
+// each: 315 and 300; 2.1M and 5.0: 634 and 697; the filter of a scan's queue, 20
+// each: 168 and 439.
+constexpr unsigned long long kCfPairs = 4ull;
+__device__ __forceinline__ bool perPoint(const RefineScratch& r) { return r.ctr->pairs < kCfPairs * r.ctr->voxels; }
+
 __global__ void __launch_bounds__(256) k_cf_index(Dev d, RefineScratch r) {
     const uint32_t nodes = r.ctr->nodes, total = r.ctr->voxels;
+    const bool direct = perPoint(r);
     // each filtered node's next filtered node up that has voxels
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nodes; k += gridDim.x * blockDim.x) {
         const uint32_t node = r.voxNode[k];
@@ -149,7 +161,7 @@ __global__ void __launch_bounds__(256) k_cf_index(Dev d, RefineScratch r) {
         if (phys != kNone) v = reinterpret_cast<const Point*>(d.arena + (uint64_t)phys * 16u)[s % d.ppc];
         const unsigned long long key = ((unsigned long long)lo << 21) | voxelCell(d, node, v);
         r.acc[e] = make_ulonglong4(0ull, 0ull, 0ull, 0ull);
-        r.up[e] = make_ulonglong4(0ull, 0ull, 0ull, 0ull);
+        if (!direct) r.up[e] = make_ulonglong4(0ull, 0ull, 0ull, 0ull);
         r.entrySlot[e] = kNone;
         if (phys == kNone) continue;
         uint32_t slot = slotOf(key, r.hashMask);
@@ -189,7 +201,7 @@ __device__ __forceinline__ uint32_t unitPoints(uint32_t ppc) { return ppc >= kCf
 __global__ void __launch_bounds__(256) k_cf_units(Dev d, RefineScratch r) {
     const uint32_t nn = d.ctr->numNodes, unit = unitPoints(d.ppc);
     const bool arenaFull = (d.ctr->overflowFlags & (uint32_t)kOvfArena) != 0u;
-    unsigned long long visited = 0;
+    unsigned long long visited = 0, pairs = 0;
     for (uint32_t leaf = blockIdx.x * blockDim.x + threadIdx.x; leaf < nn; leaf += gridDim.x * blockDim.x) {
         const uint32_t np = min(d.numPoints[leaf], d.numPointChunks[leaf] * d.ppc);
         if (np == 0u) continue;
@@ -197,12 +209,12 @@ __global__ void __launch_bounds__(256) k_cf_units(Dev d, RefineScratch r) {
         const int4 a = row[0], b = row[1];
         if ((a.x & a.y & a.z & a.w & b.x & b.y & b.z & b.w) != -1) continue;
         const uint32_t lv = d.level[leaf];
-        uint32_t m = 0, withVoxels = 0;
+        uint32_t m = 0, withVoxels = 0;  // filtered nodes, and those with voxels
         for (uint32_t l = 0; l <= lv; l++) {
             const uint32_t k = r.refSlot[l < lv ? d.anc[(size_t)leaf * kMaxDepth + l].x : leaf];
             if (k == kNone) continue;
             m++;
-            withVoxels |= r.voxBase[k + 1u] - r.voxBase[k];
+            withVoxels += r.voxBase[k + 1u] != r.voxBase[k];
         }
         uint32_t held = np;
         if (arenaFull && m > 0u) {  // points whose chunk the arena had no room for are not there
@@ -211,13 +223,20 @@ __global__ void __launch_bounds__(256) k_cf_units(Dev d, RefineScratch r) {
                 if (d.tablePool[off + k] == kNone) held -= min(d.ppc, np - k * d.ppc);
         }
         visited += (unsigned long long)held * m;
+        pairs += (unsigned long long)held * withVoxels;
         if (withVoxels == 0u) continue;
         const uint32_t units = (np + unit - 1u) / unit, first = atomicAdd(&r.ctr->units, units);
         d.accumItem[leaf] = first;
         for (uint32_t u = first; u < first + units && u < d.accumUnitCap; u++) d.accumUnitW[u] = leaf;
     }
-    for (int o = 16; o > 0; o >>= 1) visited += __shfl_xor_sync(0xFFFFFFFFu, visited, o);
-    if ((threadIdx.x & 31u) == 0 && visited) atomicAdd(&r.ctr->points, visited);
+    for (int o = 16; o > 0; o >>= 1) {
+        visited += __shfl_xor_sync(0xFFFFFFFFu, visited, o);
+        pairs += __shfl_xor_sync(0xFFFFFFFFu, pairs, o);
+    }
+    if ((threadIdx.x & 31u) == 0 && visited) {
+        atomicAdd(&r.ctr->points, visited);
+        atomicAdd(&r.ctr->pairs, pairs);
+    }
 }
 
 __device__ __forceinline__ void addSums(ulonglong4* to, unsigned long long cr, unsigned long long cg,
@@ -245,10 +264,12 @@ __global__ void __launch_bounds__(256) k_cf_gather(Dev d, RefineScratch r) {
     __shared__ uint32_t s_m;
     const uint32_t ppc = d.ppc, unit = unitPoints(ppc);
     const uint32_t units = min(r.ctr->units, d.accumUnitCap);
+    const bool direct = perPoint(r);
+    ulonglong4* alone = direct ? r.acc : r.up;  // where a point goes by itself
     for (uint32_t u = blockIdx.x; u < units; u += gridDim.x) {
         const uint32_t leaf = d.accumUnitW[u];
         const uint32_t lv = d.level[leaf];
-        for (uint32_t i = threadIdx.x; i < kCfTable; i += blockDim.x) {
+        for (uint32_t i = threadIdx.x; i < kCfTable && !direct; i += blockDim.x) {
             s_key[i] = kNone;
 #pragma unroll
             for (int k = 0; k < 4; k++) s_sum[k][i] = 0;
@@ -311,13 +332,14 @@ __global__ void __launch_bounds__(256) k_cf_gather(Dev d, RefineScratch r) {
                                z = quant28(d, p.z, 2);
                 const uint32_t color = __float_as_uint(p.w);
                 uint32_t cr = color & 255u, cg = (color >> 8) & 255u, cb = (color >> 16) & 255u, n = 1u;
-                const bool regular = max(max(x, y), z) <= (1u << 28);
+                const bool regular = !direct && max(max(x, y), z) <= (1u << 28);
                 if (there && !regular) {
                     for (uint32_t q = 0; q < m; q++) {
                         const uint32_t e = findEntry(r, ((unsigned long long)s_slot[q] << 21) | cellOf(x, y, z, s_lv[q]));
-                        if (e != kNone) addSums(&r.up[e], cr, cg, cb, 1ull);
+                        if (e != kNone) addSums(&alone[e], cr, cg, cb, 1ull);
                     }
                 }
+                if (direct) continue;
                 uint32_t cell = there && regular ? cellOf(x, y, z, top) : kNone;
                 // a warp whose points share one cell (a coarse ancestor's) adds once
                 const uint32_t cell0 = __shfl_sync(0xFFFFFFFFu, cell, 0);
@@ -347,7 +369,7 @@ __global__ void __launch_bounds__(256) k_cf_gather(Dev d, RefineScratch r) {
             }
         }
         __syncthreads();
-        for (uint32_t i = threadIdx.x; i < kCfTable; i += blockDim.x)
+        for (uint32_t i = threadIdx.x; i < kCfTable && !direct; i += blockDim.x)
             if (s_key[i] != kNone) addCell(s_key[i], s_sum[0][i], s_sum[1][i], s_sum[2][i], s_sum[3][i]);
         __syncthreads();
     }
@@ -360,6 +382,7 @@ __global__ void __launch_bounds__(256) k_cf_gather(Dev d, RefineScratch r) {
 __global__ void __launch_bounds__(256) k_cf_roll(Dev d, RefineScratch r) {
     constexpr uint32_t kAhead = 4;
     const uint32_t total = r.ctr->voxels;
+    if (perPoint(r)) return;
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
         const uint32_t slot = r.entrySlot[e];
         const ulonglong4 a = r.acc[e];
@@ -401,6 +424,7 @@ __global__ void __launch_bounds__(256) k_cf_roll(Dev d, RefineScratch r) {
 
 __global__ void __launch_bounds__(256) k_cf_apply(Dev d, RefineScratch r) {
     const uint32_t nodes = r.ctr->nodes, total = r.ctr->voxels;
+    const bool direct = perPoint(r);
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
         uint32_t lo = 0, hi = nodes;
         while (hi - lo > 1) {
@@ -410,11 +434,13 @@ __global__ void __launch_bounds__(256) k_cf_apply(Dev d, RefineScratch r) {
         }
         const uint32_t node = r.voxNode[lo], s = e - r.voxBase[lo];
         ulonglong4 a = r.acc[e];
-        const ulonglong4 up = r.up[e];
-        a.x += up.x;
-        a.y += up.y;
-        a.z += up.z;
-        a.w += up.w;
+        if (!direct) {
+            const ulonglong4 up = r.up[e];
+            a.x += up.x;
+            a.y += up.y;
+            a.z += up.z;
+            a.w += up.w;
+        }
         const uint32_t phys = d.tablePool[d.vxTableOff[node] + s / d.ppc];
         if (a.w > 0 && phys != kNone) {
             Point* v = reinterpret_cast<Point*>(d.arena + (uint64_t)phys * 16u) + s % d.ppc;
@@ -461,8 +487,8 @@ __device__ uint32_t blockExclusiveScanRefine(uint32_t v, uint32_t* total, uint32
 void launchRefineColors(const Dev& d, const RefineScratch& r, const uint32_t* queue, uint32_t queueLen,
                         uint32_t budget, int grid, cudaStream_t s) {
     k_cf_plan<<<1, 1024, 0, s>>>(d, r, queue, queueLen, budget);
-    k_cf_index<<<grid, 256, 0, s>>>(d, r);
     k_cf_units<<<grid, 256, 0, s>>>(d, r);
+    k_cf_index<<<grid, 256, 0, s>>>(d, r);
     k_cf_gather<<<grid, 256, 0, s>>>(d, r);
     k_cf_roll<<<grid, 256, 0, s>>>(d, r);
     k_cf_apply<<<grid, 256, 0, s>>>(d, r);

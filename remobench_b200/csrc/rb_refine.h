@@ -11,7 +11,8 @@ namespace rb {
 struct RefineCounters {
     uint32_t nodes;               // queue prefix filtered
     uint32_t voxels;              // accumulator entries in use
-    unsigned long long points;    // (point, filtered ancestor) pairs summed
+    unsigned long long points;    // (point, filtered ancestor) pairs
+    unsigned long long pairs;     // those whose ancestor has voxels
     uint32_t units;               // units of points the gathering pass takes
     uint32_t pad;
 };

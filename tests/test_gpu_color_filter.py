@@ -88,3 +88,31 @@ def test_sums_in_the_spill_list_and_beside_it(c1_cloud, capacity):
         compare_voxels(ctx, tree, nodes)
     ctx.close()
     tree.close()
+
+
+@pytest.mark.parametrize("points,limit,shrink", [(60_001, 300, 1.0), (60_001, 300, 0.8), (200_000, 5000, 1.0)])
+def test_cloud_that_fills_its_volume(c1_cloud, points, limit, shrink):
+    """Few points a voxel: the points go to their entries one by one."""
+    from remobench_b200.lod import make_frame
+    _, cloud, bmin, bmax = c1_cloud
+    cloud = np.ascontiguousarray(cloud[:points])
+    rng = np.random.default_rng(3)
+    for k, a in enumerate("xyz"):
+        cloud[a] = rng.uniform(bmin[k], bmax[k], points)
+    bmax = (np.asarray(bmax) * np.float32(shrink)).astype(np.float32)
+    cfg = dict(max_points_per_node=limit)
+    # more new cells a batch than the default list holds
+    ctx, _ = build_gpu(cloud, bmin, bmax, 20_011, store_capacity=4 << 30, backlog_capacity=1_000_000, **cfg)
+    tree = build_oracle(cloud, bmin, bmax, 20_011, persistent_capacity=4 << 30, **cfg)
+    f = make_frame(bmin, bmax, 1920, 1080, yaw=1.3, pitch=-0.5, radius_scale=0.5)
+    ctx.analyze(f, min_points=1, frontier_only=False, queue_capacity=16_384)
+    queue = ctx.queue()
+    for budget in (1, len(queue)):
+        r = ctx.refine_colors(budget)
+        assert (r.nodes_filtered, r.voxels_filtered) == tree.refine_colors(queue[:budget])
+        nodes = compare_nodes(ctx, tree)
+        compare_voxels(ctx, tree, nodes)
+    with_voxels = nodes["num_voxels"][queue] > 0
+    assert r.points_visited < 4 * r.voxels_filtered + int(nodes["num_points"][queue[~with_voxels]].sum())
+    ctx.close()
+    tree.close()
