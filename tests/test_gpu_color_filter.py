@@ -95,7 +95,7 @@ def test_cloud_that_fills_its_volume(c1_cloud, points, limit, shrink):
     """Few points a voxel: the points go to their entries one by one."""
     from remobench_b200.lod import make_frame
     _, cloud, bmin, bmax = c1_cloud
-    cloud = np.ascontiguousarray(cloud[:points])
+    cloud = cloud[:points].copy()
     rng = np.random.default_rng(3)
     for k, a in enumerate("xyz"):
         cloud[a] = rng.uniform(bmin[k], bmax[k], points)
