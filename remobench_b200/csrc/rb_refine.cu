@@ -190,9 +190,12 @@ __device__ __forceinline__ uint32_t findEntry(const RefineScratch& r, unsigned l
 }
 
 // The points of one unit: whole chunks, about kCfUnit points, so that a leaf
-// has no more units than chunks.
-constexpr uint32_t kCfUnit = 2048;
-__device__ __forceinline__ uint32_t unitPoints(uint32_t ppc) { return ppc >= kCfUnit ? ppc : kCfUnit / ppc * ppc; }
+// has no more units than chunks; of larger chunks no more than the 32-bit sums of
+// one cell hold (255 a point).
+constexpr uint32_t kCfUnit = 2048, kCfUnitMax = 1u << 24;
+__device__ __forceinline__ uint32_t unitPoints(uint32_t ppc) {
+    return ppc >= kCfUnit ? min(ppc, kCfUnitMax) : kCfUnit / ppc * ppc;
+}
 
 // Per node: a leaf with points below (or itself) a filtered node adds its
 // (point, filtered ancestor) pairs to the count and, where one of those has

@@ -116,3 +116,28 @@ def test_cloud_that_fills_its_volume(c1_cloud, points, limit, shrink):
     assert r.points_visited < 4 * r.voxels_filtered + int(nodes["num_points"][queue[~with_voxels]].sum())
     ctx.close()
     tree.close()
+
+
+def test_one_cell_of_17_million_points():
+    """More points in a chunk, and in one cell, than 32-bit sums of colours hold."""
+    from remobench_b200.lod import make_frame
+    n, box = 17_000_000, (np.zeros(3, np.float32), np.full(3, 128.0, np.float32))
+    cloud = np.zeros(n, dtype=np.dtype([("x", "<f4"), ("y", "<f4"), ("z", "<f4"), ("color", "<u4")]))
+    for k, a in enumerate("xyz"):
+        cloud[a] = 0.5
+        # in another octant, so that the root splits; near its corner, as the others
+        cloud[a][-100_000:] = np.random.default_rng(k).uniform(0.0, 1.0, 100_000) + (65.0 if k == 0 else 0.0)
+    cloud["color"] = 0xFF00FFFF
+    cloud["color"][0] = 0xFF000000  # the voxel's own colour, of the lowest index
+    ctx, _ = build_gpu(cloud, *box, n, points_per_chunk=20_000_000, max_points_per_node=16_950_000, backlog_capacity=200_000,
+                       store_capacity=4 << 30)
+
+    def colour():
+        v = ctx.node_voxels(0)
+        return v["color"][v["x"] == 0.5].tolist()
+    ctx.analyze(make_frame(*box, 1920, 1080, yaw=1.3, pitch=-0.5, radius_scale=0.5), min_points=1, frontier_only=False)
+    queue = ctx.queue()
+    assert 0 in queue and colour() == [0xFF000000]
+    ctx.refine_colors(len(queue))
+    assert colour() == [0xFF00FFFF]
+    ctx.close()
