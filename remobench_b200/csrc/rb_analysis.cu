@@ -54,7 +54,7 @@ __device__ __forceinline__ bool leafA(const Dev& d, uint32_t node) {
 // by the longest chain of dependent round trips, one arrival and one read per
 // level of the tree, not by bytes (184 B read and written per node). Measured
 // at 31,497 nodes: 232 us as a launch per level (a pass over all nodes for each
-// of the 21, whatever the tree's depth), 37 us so; at 2,000 nodes 120 and
+// of the 21, whatever the tree's depth), 38 us so; at 2,000 nodes 120 and
 // 23 us. Re-basing at every step of the chain instead: 59 and 33 us.
 constexpr uint32_t kRollThreads = 128;
 constexpr uint32_t kRollWords = sizeof(RollSum) / 8u;

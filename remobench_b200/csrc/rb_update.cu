@@ -1841,8 +1841,8 @@ __global__ void __launch_bounds__(256) k_vox_sample(Dev d, const Point* __restri
                 else atomicCAS(&d.hashSlots[slot].y, kHashEmpty, val);
             }
         }
-        // claimed slots wait in the warp's buffer; 32 or more go to the list of
-        // new cells with one counter atomic
+        // claimed slots wait in the warp's buffer; kWarpFlush or more go to the list
+        // of new cells with one counter atomic
         const unsigned cm = __ballot_sync(0xFFFFFFFFu, claimed);
         if (claimed) wbuf[wbufN + (uint32_t)__popc(cm & ((1u << lane) - 1u))] = slot;
         __syncwarp();
